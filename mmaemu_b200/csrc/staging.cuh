@@ -1,0 +1,106 @@
+// Device code shared by the kernels that work on 128 x 128 output tiles and 32-wide k-tiles (kernel_fast.cu):
+// tile numbering, the codes a thread decodes, mbarriers and bulk copies, and the power base of the exponent pass.
+#pragma once
+#include "common.cuh"
+#include "fast_math.cuh"
+
+namespace mmb {
+namespace {
+
+constexpr int BM = 128, BN = 128, KT = 32, THREADS = 256;
+
+// The power base of a format pair's tensor-core exponent pass (2^8, 2^5 or 2^4 per unit of exponent): see
+// block_strip_mma and fast_math.cuh.
+__host__ __device__ constexpr int tc_pow_mul(int fa, int fb) {
+  return (fa == MMB200_FMT_E4M3 && fb == MMB200_FMT_E4M3) ? 8 : ((fa == MMB200_FMT_E5M2 && fb == MMB200_FMT_E5M2) ? 4 : 5);
+}
+
+// Output tile of a CTA. Tiles are numbered in bands of BAND tile columns, row by row inside a band, so that the CTAs that
+// run at the same time share a band of B tiles that stays in L2 (a band of 16 decoded tile columns of K = 4096 is about
+// 70 MB) while the A tiles stream through once per band.
+constexpr int BAND = 16;
+__device__ __forceinline__ void tile_of_cta(const Params& p, int idx, int& tile_m, int& tile_n) {
+  const int per_band = BAND * p.tiles_m, b = idx / per_band, rem = idx - b * per_band;
+  const int w = min(BAND, p.tiles_n - b * BAND);
+  tile_m = rem / w;
+  tile_n = b * BAND + rem % w;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// Quantise prologue (the scalar conversion is fm::quantise_e4m3 in fast_math.cuh).
+// The 16 codes of row `row` starting at element k of one operand: the caller's FP8 codes, or -- operand A with the
+// quantise prologue -- the codes of 16 activations, which are also written to the codes array.
+template <bool IS_A>
+__device__ __forceinline__ uint4 load_codes16(const Params& p, int row, int rows, int k) {
+  if (row >= rows || k >= p.K) return make_uint4(0, 0, 0, 0);
+  if (!IS_A || !p.a_hp)
+    return __ldg(reinterpret_cast<const uint4*>((IS_A ? p.A : p.B) + (long long)row * (IS_A ? p.lda : p.ldb) + k));
+  const float scale = __ldg(p.a_quant_scale);
+  float x[16];
+  if (p.a_hp_dtype == MMB200_HP_F32) {
+    const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(p.a_hp) + (long long)row * p.ld_hp + k);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float4 f = __ldg(src + q);
+      x[4 * q] = __fmul_rn(f.x, scale); x[4 * q + 1] = __fmul_rn(f.y, scale);
+      x[4 * q + 2] = __fmul_rn(f.z, scale); x[4 * q + 3] = __fmul_rn(f.w, scale);
+    }
+  } else {                        // bf16: torch multiplies in bf16 -- the scale and the product are rounded to bf16
+    const float scale_b = __uint_as_float((uint32_t)f32_to_bf16_bits(scale) << 16);
+    const uint4* src = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.a_hp) + (long long)row * p.ld_hp + k);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const uint4 w = __ldg(src + q);
+      const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const float lo = __fmul_rn(__uint_as_float(ws[h] << 16), scale_b);
+        const float hi = __fmul_rn(__uint_as_float(ws[h] & 0xFFFF0000u), scale_b);
+        x[8 * q + 2 * h] = __uint_as_float((uint32_t)f32_to_bf16_bits(lo) << 16);
+        x[8 * q + 2 * h + 1] = __uint_as_float((uint32_t)f32_to_bf16_bits(hi) << 16);
+      }
+    }
+  }
+  uint32_t w4[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    w4[q] = fm::quantise_e4m3(x[4 * q]) | (fm::quantise_e4m3(x[4 * q + 1]) << 8) | (fm::quantise_e4m3(x[4 * q + 2]) << 16) |
+            (fm::quantise_e4m3(x[4 * q + 3]) << 24);
+  const uint4 codes = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+  *reinterpret_cast<uint4*>(p.a_codes + (long long)row * p.lda + k) = codes;
+  return codes;
+}
+
+__device__ __forceinline__ uint32_t smem_addr(const void* ptr) { return (uint32_t)__cvta_generic_to_shared(ptr); }
+
+constexpr int WAIT_POLLS = 1 << 22;        // default bound of every mbarrier wait (each poll suspends for up to ~1 us)
+
+__device__ __forceinline__ void mbar_init(unsigned long long* bar, int count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count));
+}
+__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+// Bounded wait for the phase with the given parity: at most `polls` polls. Returns false if the bound ran out.
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, uint32_t parity, int polls) {
+  const uint32_t addr = smem_addr(bar);
+  for (int i = 0; i < polls; ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+    if (done) return true;
+  }
+  return false;
+}
+// Bulk copy global -> shared (both 16-byte aligned, size a multiple of 16), completion counted on `bar`.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, unsigned long long* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar)) : "memory");
+}
+
+}  // namespace
+}  // namespace mmb

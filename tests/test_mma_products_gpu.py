@@ -1,0 +1,67 @@
+"""The tensor-core block step against the integer kernel, where its instruction's rounding decides the result.
+
+The staged kernels let mma.sync cut every product: an accumulator of +-1.5 * 2^(E+12) makes the instruction truncate each
+of its 16 summands toward zero at 2^(E-13), the model's unit (kernel_fast.cu, block_strip_mma). Here every pair of codes
+of a format pair is multiplied under block exponents that move across its bits, given by another product of the block and,
+from the second block on, by the accumulator; the integer kernel, which shares no arithmetic with it, gives the expected
+bits. Everything is bit-exact: no tolerance."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+PAIRS = (("e4m3", "e4m3"), ("e5m2", "e4m3"), ("e4m3", "e5m2"), ("e5m2", "e5m2"))
+
+
+def powers(fmt):
+    """Codes of +2^e for every normal and subnormal power of two of a format."""
+    return np.array([1, 2, 4] + [e << 3 for e in range(1, 16)], np.uint8) if fmt == "e4m3" else \
+        np.array([1, 2] + [e << 2 for e in range(1, 31)], np.uint8)
+
+
+def finite_codes(fmt):
+    c = np.arange(256, dtype=np.uint8)
+    return c[(c & 0x7F) != 0x7F] if fmt == "e4m3" else c[(c & 0x7C) != 0x7C]
+
+
+def same(a, b, **kw):
+    import gpu_runner
+    got = gpu_runner.accumulate(a, b, kernel="staged", **kw)
+    want = gpu_runner.accumulate(a, b, kernel="integer", **kw)
+    bad = np.argwhere(got != want)
+    assert bad.size == 0, f"{len(bad)} of {got.size} differ, first {bad[0]}: {got[tuple(bad[0])]:#x} != " \
+                          f"{want[tuple(bad[0])]:#x}"
+
+
+@pytest.mark.parametrize("preset", (16, 32))
+@pytest.mark.parametrize("fmts", PAIRS, ids="x".join)
+def test_every_code_pair_under_every_block_exponent(fmts, preset):
+    """Rows: all codes of A; columns: all codes of B. One product a * b per block, at a varying place of the block, beside
+    an anchor product 2^e that sets the block exponent; a second, negated copy three blocks later meets an accumulator."""
+    ca, cb = finite_codes(fmts[0]), finite_codes(fmts[1])
+    pa, pb = powers(fmts[0]), powers(fmts[1])
+    for n, anchor in enumerate([(x, pb[-1]) for x in pa] + [(pa[0], y) for y in pb]):
+        a, b = np.zeros((ca.size, 128), np.uint8), np.zeros((cb.size, 128), np.uint8)
+        place = (5 * n) % 16
+        a[:, place], b[:, place] = ca, cb
+        a[:, (place + 7) % 16], b[:, (place + 7) % 16] = anchor
+        a[:, 96 + place], b[:, 96 + place] = ca ^ 0x80, cb
+        same(a, b, fmt_a=fmts[0], fmt_b=fmts[1], preset=preset, fast=True)
+
+
+@pytest.mark.parametrize("preset", (16, 32))
+@pytest.mark.parametrize("fmts", PAIRS, ids="x".join)
+def test_blocks_full_of_cut_products(fmts, preset):
+    """Random blocks over the full range of exponents: most products lose bits, sums and accumulators change sign; and
+    blocks of the largest products of one sign, where the block sum comes closest to the edge of the offset's binade."""
+    rng = np.random.default_rng(7 + preset)
+    ca, cb = finite_codes(fmts[0]), finite_codes(fmts[1])
+    same(rng.choice(ca, (256, 512)), rng.choice(cb, (256, 512)), fmt_a=fmts[0], fmt_b=fmts[1], preset=preset, fast=True)
+    top_a, top_b = (0x7E if f == "e4m3" else 0x7B for f in fmts)
+    a = np.full((128, 256), top_a, np.uint8)
+    b = np.full((128, 256), top_b, np.uint8)
+    a[:, 128:] ^= 0x80
+    a[1::2] ^= 0x80
+    a[::3, ::5] = rng.choice(ca, a[::3, ::5].shape)
+    same(a, b, fmt_a=fmts[0], fmt_b=fmts[1], preset=preset, fast=True)
+    same(a, b, fmt_a=fmts[0], fmt_b=fmts[1], preset=preset, fast=False)
