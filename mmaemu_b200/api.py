@@ -302,8 +302,10 @@ def _workspace(L, kernel: str, a_ptr, lda, b_ptr, ldb, M, N, K, nfma, S, device)
     comes from torch's caching allocator, which hands it out again only to later work on the same stream."""
     if kernel in ("integer", "direct") or os.environ.get("MMAEMU_B200_WORKSPACE", "1") == "0":
         return None, None, 0
-    if L.mmb200_kernel_for(a_ptr, lda, b_ptr, ldb, K, nfma, 1) != _lib.KERNEL_CODES["fast"]:
-        return None, None, 0                 # operands the fast kernels cannot read: the integer kernel serves the call
+    if kernel != "auto" and L.mmb200_kernel_for(a_ptr, lda, b_ptr, ldb, K, nfma, 1) != _lib.KERNEL_CODES["fast"]:
+        return None, None, 0                 # operands the fast kernels cannot read with 16-byte loads
+    if nfma not in (16, 32):
+        return None, None, 0                 # the late-accumulator preset runs on the integer kernel
     n = int(L.mmb200_workspace_bytes_split(M, N, K, S))
     if S > 1 and n > SPLIT_WORKSPACE_LIMIT:
         return None, None, 0                 # split plans keep 8 bytes of scratch per output; very large ones run on the integer kernel

@@ -16,10 +16,10 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libmmaemu_b200.so"
-SOURCES = ("api.cu", "kernel_integer.cu", "kernel_fast.cu", "static_scratch.cu")
+SOURCES = ("api.cu", "kernel_integer.cu", "kernel_fast.cu", "kernel_umma.cu", "static_scratch.cu")
 # translation units: (source, extra defines). kernel_fast.cu is compiled once per FP8 format pair and kind of kernel
 # (tensor cores: parts 0..3, CUDA cores: 4..7), in parallel.
-UNITS = (("api.cu", ()), ("kernel_integer.cu", ()), ("static_scratch.cu", ()),
+UNITS = (("api.cu", ()), ("kernel_integer.cu", ()), ("static_scratch.cu", ()), ("kernel_umma.cu", ()),
          *(("kernel_fast.cu", (f"-DMMB_PART={part}",)) for part in range(8)))
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "--fmad=false", "-std=c++17",
               "-Xcompiler", "-fPIC"]

@@ -83,6 +83,9 @@ struct Params {
   int slice_start[MMB200_MAX_SLICES + 1];
   int chain_base[MMB200_MAX_SLICES + 1];
   float* ws_chains;
+  int byte_loads;        // the operands cannot be read with 16-byte loads (staged kernels: they read single codes)
+  int umma;              // the launch runs on the tcgen05 kernels: chain results are laid out [column][row] per tile
+  int wide_tiles;        // tcgen05, unsplit: 256 columns per CTA instead of 128
 };
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -279,10 +282,13 @@ struct Epilogue {
 // Launchers implemented by the kernel translation units; each returns a cudaError_t.
 cudaError_t launch_integer(const Params& p, int nfma, cudaStream_t stream);
 cudaError_t launch_fast(const Params& p, int nfma, cudaStream_t stream);
+// tcgen05 kernels (kernel_umma.cu), called by the staged launches: operand images, then the GEMM; p filled in by them.
+cudaError_t launch_umma(const Params& p, int nfma, cudaStream_t stream, int* launches);
 bool fast_supports(const Params& p, int nfma);
 // Staged fast kernel: scratch bytes it needs for a shape, and the launch (pre-decode of both operands, then the GEMM).
 // `launches` is increased by the number of kernels launched.
-bool staged_supports(const Params& p, int nfma);            // like fast_supports, any plan
+bool staged_supports(const Params& p, int nfma);            // any plan, any operands (with scratch memory)
+bool staged_vector_supports(const Params& p, int nfma);     // any plan, operands that 16-byte loads can read
 size_t staged_workspace_bytes(int M, int N, int K, int S, bool with_slices, bool shared_b = false);
 // Bytes of a shared B area (tile images of every 128-column group, then one int per column), and the launch that fills
 // it (p.B, p.ldb, p.N, p.K, the formats; p.shared_b = the area, 128-byte aligned).

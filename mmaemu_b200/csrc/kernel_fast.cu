@@ -572,7 +572,9 @@ __global__ void __launch_bounds__(THREADS) combine_kernel(const __grid_constant_
   int tile_m, tile_n;
   tile_of_cta(p, (int)blockIdx.x, tile_m, tile_n);
   const Lane ln(tid);
-  const int gm = tile_m * BM + ln.row(i), gn = tile_n * BN + ln.col(j);
+  // the position of a chain result in its tile: by the threads of the first pass, or [column][row] (tcgen05 kernels)
+  const int lin = idx * THREADS + tid;
+  const int gm = tile_m * BM + (p.umma ? lin % BM : ln.row(i)), gn = tile_n * BN + (p.umma ? lin / BM : ln.col(j));
   if (gm >= p.M || gn >= p.N) return;
   if (p.status && *reinterpret_cast<volatile int*>(p.status)) return;   // a slice gave up waiting: no output, as in the other modes
   const float* src = p.ws_chains + (size_t)blockIdx.x * p.n_chains * (TM * TN * THREADS) + (size_t)idx * THREADS + tid;
@@ -780,36 +782,15 @@ __global__ void __launch_bounds__(THREADS) predecode_kernel(const __grid_constan
   if (cls) atomicOr(&flags[row], (int)cls);
 }
 
-// fp16 pair words of the 4 sanitised codes of a word (exact).
-template <int FMT>
-__device__ __forceinline__ void code_halves(uint32_t ws, uint32_t& h01, uint32_t& h23) {
-  if (FMT == MMB200_FMT_E4M3) {
-    asm("{.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, lo;\n\tcvt.rn.f16x2.e4m3x2 %1, hi;}"
-        : "=r"(h01), "=r"(h23) : "r"(ws));
-  } else {                                                       // an E5M2 code is the high byte of an fp16
-    h01 = __byte_perm(ws, 0u, 0x1404);
-    h23 = __byte_perm(ws, 0u, 0x3424);
-  }
-}
-
 // Decodes 16 codes of one row (k = 16 lhalf .. + 15 of the k-tile) into a tile of the tensor-core kernels; returns the
 // non-finite classes seen.
 template <int FA, int FB, bool IS_A, class Tile>
 __device__ __forceinline__ uint32_t decode16_tc(const uint4 raw, Tile& tile, int lrow, int lhalf) {
-  constexpr int FMT = IS_A ? FA : FB, POWMUL = tc_pow_mul(FA, FB);
-  constexpr uint32_t POW_BIAS = POWMUL == 8 ? (IS_A ? fm::POW_BIAS_A : fm::POW_BIAS_B)
-                                            : (POWMUL == 5 ? fm::POW5_BIAS : (IS_A ? fm::POW4_BIAS_A : fm::POW4_BIAS_B));
-  const uint32_t w4[4] = {raw.x, raw.y, raw.z, raw.w};
-  uint32_t seen = 0, v0[4], v1[4];
+  uint32_t w4[4] = {raw.x, raw.y, raw.z, raw.w}, seen = 0, v0[4], v1[4];
 #pragma unroll
   for (int w = 0; w < 4; ++w) {
-    uint32_t ws, xb, tc, sg, cls, pw;
-    fm::decode_bits<FMT, POWMUL>(w4[w], 0, 0, 0, ws, xb, tc, sg, cls, &pw, POW_BIAS);
-    seen |= cls;
-    code_halves<FMT>(ws, v0[w], v1[w]);                          // k = 16 lhalf + 4 w .. + 3: words s = 4 lhalf + w of h = 0, 1
-    // bf16 with exponent field pw and zero mantissa: field << 7
-    const uint32_t lo = ((pw & 0xFFu) << 7) | ((pw & 0xFF00u) << 15);
-    const uint32_t hi = (((pw >> 16) & 0xFFu) << 7) | (((pw >> 16) & 0xFF00u) << 15);
+    uint32_t lo, hi;
+    decode4<FA, FB, IS_A>(w4[w], v0[w], v1[w], lo, hi, seen);    // k = 16 lhalf + 4 w .. + 3: words s = 4 lhalf + w of h = 0, 1
     *(reinterpret_cast<uint2*>(&tile.e[lrow][chunk_at(lrow, w)]) + lhalf) = make_uint2(lo, hi);
   }
   tile.v[lrow][chunk_at(lrow, lhalf)] = make_uint4(v0[0], v0[1], v0[2], v0[3]);
@@ -1209,6 +1190,11 @@ cudaError_t launch_alu_e5m2_e5m2(const Params&, int, cudaStream_t, bool, int*);
 
 namespace {
 
+// Every pair but E5M2 x E5M2 (whose exponent pass needs 8-term sums) can run on tcgen05: unsplit plans, and K slices of any.
+bool umma_supports(const Params& p) {
+  return !p.no_tensor_epass && !(p.fmt_a == MMB200_FMT_E5M2 && p.fmt_b == MMB200_FMT_E5M2);
+}
+
 cudaError_t dispatch_formats(const Params& p, int nfma, cudaStream_t stream, bool staged, int* launches) {
   const int pair = p.fmt_a * 2 + p.fmt_b;
   if (staged && !p.no_tensor_epass) {
@@ -1229,8 +1215,6 @@ cudaError_t dispatch_formats(const Params& p, int nfma, cudaStream_t stream, boo
 
 // K slicing is worth its second pass when the output tiles leave most SMs idle; it aims at about two CTAs per SM.
 constexpr int SLICE_TILE_LIMIT = 74, SLICE_CTA_TARGET = 296;
-constexpr int ROW_GROUP_COST = 260;   // time of a 16-row CTA in thousandths of the time of a 128-row CTA over the same k
-constexpr int ROW_GROUP_COST2 = 364;  // the same for two of them sharing an SM (each runs 1.4 times longer)
 constexpr size_t SLICE_SCRATCH_LIMIT = (size_t)4 << 30;
 
 struct WorkspaceLayout {
@@ -1274,17 +1258,18 @@ WorkspaceLayout workspace_layout(int M, int N, int K, int S, bool with_slices, b
 
 }  // namespace
 
-// The fast kernels read operands with 16-byte loads. Without scratch memory they serve unsplit plans only; the staged
-// kernels walk every plan.
-bool staged_supports(const Params& p, int nfma) {
-  if (nfma != 16 && nfma != 32) return false;
-  if (p.S < 1 || p.S > MMB200_MAX_SPLITS) return false;
-  if (p.K <= 0 || (p.K % 16) != 0) return false;
-  if ((reinterpret_cast<uintptr_t>(p.A) | reinterpret_cast<uintptr_t>(p.B)) & 15) return false;
-  if ((p.lda | p.ldb) & 15) return false;
-  return true;
+// Without scratch memory the fast kernels read operands with 16-byte loads and serve unsplit plans only; the staged kernels
+// walk every plan and read any operand (single codes where 16-byte loads do not fit).
+namespace {
+bool vector_loads(const Params& p) {
+  return (p.K % 16) == 0 && !((reinterpret_cast<uintptr_t>(p.A) | reinterpret_cast<uintptr_t>(p.B)) & 15) && !((p.lda | p.ldb) & 15);
 }
-bool fast_supports(const Params& p, int nfma) { return p.S == 1 && staged_supports(p, nfma); }
+}  // namespace
+bool staged_supports(const Params& p, int nfma) {
+  return (nfma == 16 || nfma == 32) && p.S >= 1 && p.S <= MMB200_MAX_SPLITS && p.K > 0;
+}
+bool fast_supports(const Params& p, int nfma) { return p.S == 1 && staged_supports(p, nfma) && vector_loads(p); }
+bool staged_vector_supports(const Params& p, int nfma) { return staged_supports(p, nfma) && vector_loads(p); }
 
 cudaError_t launch_fast(const Params& p_in, int nfma, cudaStream_t stream) {
   Params p = p_in;
@@ -1333,6 +1318,7 @@ cudaError_t launch_predecode_b(const Params& p_in, int nfma, cudaStream_t stream
   }
   cudaError_t err = cudaMemsetAsync(p.ws_flag_b, 0, (size_t)w.tiles_n * BN * sizeof(int), stream);
   if (err != cudaSuccess) return err;
+  if (p.S <= 1 && umma_supports(p)) return launch_umma(p, nfma, stream, launches);   // as launch_staged decides for a shared B area
   return dispatch_formats(p, nfma, stream, true, launches);
 }
 
@@ -1390,32 +1376,50 @@ cudaError_t launch_staged(const Params& p_in, int nfma, void* workspace, size_t 
       const size_t need = (size_t)tiles * (size_t)chains * TM * TN * THREADS * sizeof(float);
       return (n >= 2 && need <= wx.chains_bytes) ? n : 1;
     };
-    int slices = slices_for(rows16 ? tiles16 : tiles);
-    // Row groups: when the 128 x 128 tiles and the chains of the plan leave most SMs without a CTA, the 16-row kernels
-    // take the call -- up to eight CTAs per tile, each doing an eighth of a tile's work at about half the efficiency
-    // (ROW_GROUP_COST per mille of a tile's time), two of them per SM. The estimate compares waves of CTAs on the
-    // device's SMs. The 16-row
-    // kernels walk unsplit plans in one pass and any plan in K slices, so a split plan needs at least two slices.
-    if (!rows16 && !p.a_hp && !env_off("MMAEMU_B200_ROW_GROUPS")) {
+    // Kernel choice by estimated time, in microseconds per k-tile of 32 and wave of CTAs (measured on whole calls at K = 4096,
+    // overheads taken off): a 16-row CTA, alone on an SM or two sharing it; a 128 x 128 tile on tcgen05 (16 / 32 products
+    // per block) or on mma.sync; 256 columns per tcgen05 CTA. K slices add two launches (SLICE_LAUNCH) and, per chain, the
+    // traffic of the chain results.
+    const long long sms = sm_count();
+    const bool umma_any = umma_supports(p) && !(shared_b && p.S > 1), umma_whole = umma_any && p.S == 1;
+    const double ROWS16 = nfma == 32 ? 0.95 : 1.25, ROWS16_PAIR = nfma == 32 ? 1.35 : 1.75, SLICE_LAUNCH = 8.0;
+    const bool one_sum = nfma == 16 || (p.fmt_a == MMB200_FMT_E4M3 && p.fmt_b == MMB200_FMT_E4M3);
+    const double UMMA = nfma == 16 ? 2.2 : (one_sum ? 1.3 : 1.65), MMA = nfma == 16 ? 3.3 : 3.0, PREDECODE = 12.0;
+    auto waves16 = [&](long long n) {
+      const long long pairs = n / (2 * sms), rest = n % (2 * sms);
+      return pairs * ROWS16_PAIR + (rest == 0 ? 0.0 : (rest <= sms ? ROWS16 : ROWS16_PAIR));
+    };
+    auto sliced = [&](double per_tile, int n) { return per_tile * w.k_tiles / n + (n > 1 ? SLICE_LAUNCH : 0.0); };
+    const int s128 = slices_for(tiles);
+    const double umma_tile = (double)((tiles * s128 + sms - 1) / sms) * (umma_any ? UMMA : MMA);
+    const double time128 = sliced(umma_tile, s128) + PREDECODE;
+    int slices = s128;
+    // calls of at most 16 rows always; others when the estimate says so: up to eight CTAs per tile, each decoding B itself
+    if (rows16 || (!p.a_hp && !env_off("MMAEMU_B200_ROW_GROUPS"))) {
       int s16 = slices_for(tiles16);
       if (p.S > 1 && s16 < 2 && can_slice && chains >= 2 &&
           (size_t)tiles * (size_t)chains * TM * TN * THREADS * sizeof(float) <= wx.chains_bytes)
         s16 = 2;
-      const long long sms = sm_count();
-      const long long waves8 = (tiles * slices + sms - 1) / sms;
-      // two 16-row CTAs share an SM: a full double wave costs ROW_GROUP_COST2, a last wave of at most one CTA per SM
-      // ROW_GROUP_COST
-      const long long n16 = tiles16 * s16, pairs = n16 / (2 * sms), rest = n16 % (2 * sms);
-      const long long units16 = pairs * ROW_GROUP_COST2 + (rest == 0 ? 0 : (rest <= sms ? ROW_GROUP_COST : ROW_GROUP_COST2));
-      // time in units of (one tile over all of K) / 1000: a slice does 1 / slices of it
-      const long long time8 = waves8 * 1000 / slices, time16 = units16 / s16;
-      if ((p.S == 1 || s16 >= 2) && time16 * 10 < time8 * 9) {
+      // a short unsplit problem is done before the launches of a second pass would be
+      if (p.S == 1 && s16 > 1 && sliced(waves16(tiles16), 1) < sliced(waves16(tiles16 * s16), s16)) s16 = 1;
+      const double time16 = sliced(waves16(tiles16 * s16), s16);
+      if (rows16 || ((p.S == 1 || s16 >= 2) && time16 < 0.95 * time128)) {
+        slices = rows16 && p.S > 1 && s16 < 2 ? s128 : s16;
+        p.row_groups = rows16 ? 1 : 8;
         rows16 = true;
-        slices = s16;
-        p.row_groups = 8;
       }
     }
+    // the tiles of a shared B area are images for one kind of kernel, chosen without M: no K slices of 128-row tiles then
+    if (shared_b && !rows16 && umma_whole) slices = 1;
     p.few_rows = rows16 ? 1 : 0;
+    p.umma = !rows16 && umma_any && (p.S == 1 || slices > 1);
+    if (slices > 1)
+      for (uint32_t entry : seq)
+        if (entry & SEQ_EMPTY) p.umma = 0;     // splits without k-tiles: the general walkers
+    // 256 columns per CTA (fast accumulation, one exponent sum): 1.75 times a 128-column tile's time, and fewer, longer waves
+    const long long wide = (long long)w.tiles_m * ((w.tiles_n + 1) / 2);
+    p.wide_tiles = p.umma && slices == 1 && p.fast && one_sum &&
+                   (double)((wide + sms - 1) / sms) * 1.75 < (double)((tiles + sms - 1) / sms);
     if (slices >= 2) {
       w = wx;
       p.slices = slices;
@@ -1434,6 +1438,7 @@ cudaError_t launch_staged(const Params& p_in, int nfma, void* workspace, size_t 
     p.ws_flag_b = reinterpret_cast<int*>(p.shared_b + shared_b_flags_offset(p.N, p.K));
   }
   p.only_b = 0;
+  p.byte_loads = vector_loads(p) ? 0 : 1;
   p.status = reinterpret_cast<int*>(base + w.status);
   p.plan_group = plan.group;
   p.wait_polls = g_wait_polls.load();
@@ -1459,6 +1464,14 @@ cudaError_t launch_staged(const Params& p_in, int nfma, void* workspace, size_t 
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     *launches += 1;
+  }
+  if (p.umma) {
+    err = launch_umma(p, nfma, stream, launches);
+    if (err != cudaSuccess || p.slices == 1) return err;
+    combine_kernel<<<dim3((unsigned)(w.tiles_m * w.tiles_n), TM * TN), THREADS, 0, stream>>>(p);
+    err = cudaGetLastError();
+    if (err == cudaSuccess) *launches += 1;
+    return err;
   }
   return dispatch_formats(p, nfma, stream, true, launches);
 }
