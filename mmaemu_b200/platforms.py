@@ -12,11 +12,13 @@ query on the profile's own GPU" step does not exist here (matches_device is alwa
 from __future__ import annotations
 
 import os
+import functools
 from dataclasses import dataclass
 
 DEFAULT_PROFILE = "hopper"
 
 
+@functools.lru_cache(maxsize=64)
 def _dtype_name(dt):
     if dt is None:
         return None

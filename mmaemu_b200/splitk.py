@@ -18,6 +18,7 @@ UnvalidatedEnvelopeWarning. `dry=True` (explain) warns every time and does not u
 """
 from __future__ import annotations
 
+import bisect
 import hashlib
 import json
 import os
@@ -103,6 +104,9 @@ class SplitTable:
         order = np.lexsort((shape, setting))
         self._setting, self._shape = setting[order], shape[order]
         self._splits, self._custom = z["splitK"][order], z["custom"][order]
+        # rows of every setting: [first, end) in the sorted arrays
+        values, first, counts = np.unique(self._setting, return_index=True, return_counts=True)
+        self._range = {int(v): (int(f), int(f + n)) for v, f, n in zip(values, first, counts)}
         self._settings = {(int(s["ws"]), s["out"], bool(s["fast"]), s["fmt_a"], s["fmt_b"]): s
                           for s in self.meta["settings"]}
         self.verified = {(bool(c[0]), int(c[1]), c[2], c[3], c[4]) for c in self.meta["verified_combos"]}
@@ -140,12 +144,12 @@ class SplitTable:
             return None
         s = ((self.ws_values.index(ws) << 16) | (OUT_CODES[out] << 8) | (int(bool(fast)) << 4)
              | (FMT_CODES[fmt_a] << 2) | FMT_CODES[fmt_b])
-        lo, hi = np.searchsorted(self._setting, s, "left"), np.searchsorted(self._setting, s, "right")
-        if lo == hi:
+        rows = self._range.get(s)
+        if rows is None:
             return None
         key = (int(M) << 42) | (int(N) << 21) | int(K)
-        i = lo + int(np.searchsorted(self._shape[lo:hi], key))
-        if i >= hi or int(self._shape[i]) != key:
+        i = bisect.bisect_left(self._shape, key, rows[0], rows[1])      # (np.searchsorted on a slice: 3 us more per call)
+        if i >= rows[1] or int(self._shape[i]) != key:
             return None
         return {"splitK": int(self._splits[i]), "custom": int(self._custom[i])}
 
