@@ -253,6 +253,30 @@ struct Epilogue {
     else if (es == 2) *reinterpret_cast<uint16_t*>(dst) = (uint16_t)b;
     else *dst = (uint8_t)b;
   }
+  // The same for CNT (8 or 16) consecutive columns of one row, packed into 16- or 8-byte stores (rows are 17 16-byte pieces
+  // apart for 16-bit outputs, so 32 lanes with a row each cover all banks).
+  template <int CNT>
+  __device__ __forceinline__ void park_row(unsigned char* tile, int lr, int lc, const float (&v)[CNT]) const {
+    const int es = elem_size();
+    unsigned char* dst = tile + lr * tile_pitch() + lc * es;
+    uint32_t b[CNT];
+#pragma unroll
+    for (int q = 0; q < CNT; ++q) b[q] = bits_of(v[q]);
+    if (es == 4) {
+#pragma unroll
+      for (int q = 0; q < CNT; q += 4) *reinterpret_cast<uint4*>(dst + 4 * q) = make_uint4(b[q], b[q + 1], b[q + 2], b[q + 3]);
+    } else if (es == 2) {
+#pragma unroll
+      for (int q = 0; q < CNT; q += 8)
+        *reinterpret_cast<uint4*>(dst + 2 * q) = make_uint4(b[q] | (b[q + 1] << 16), b[q + 2] | (b[q + 3] << 16),
+                                                            b[q + 4] | (b[q + 5] << 16), b[q + 6] | (b[q + 7] << 16));
+    } else {
+#pragma unroll
+      for (int q = 0; q < CNT; q += 8)
+        *reinterpret_cast<uint2*>(dst + q) = make_uint2(b[q] | (b[q + 1] << 8) | (b[q + 2] << 16) | (b[q + 3] << 24),
+                                                        b[q + 4] | (b[q + 5] << 8) | (b[q + 6] << 16) | (b[q + 7] << 24));
+    }
+  }
   // `rows`: how many rows of the image (from its first) were parked
   __device__ __forceinline__ void flush(const Params& p, const unsigned char* tile, int m0, int n0, int tid,
                                         int nthreads, int rows = TILE_DIM) const {

@@ -1416,10 +1416,12 @@ cudaError_t launch_staged(const Params& p_in, int nfma, void* workspace, size_t 
     if (slices > 1)
       for (uint32_t entry : seq)
         if (entry & SEQ_EMPTY) p.umma = 0;     // splits without k-tiles: the general walkers
-    // 256 columns per CTA (fast accumulation, one exponent sum): 1.75 times a 128-column tile's time, and fewer, longer waves
+    // 256 columns per CTA (one exponent sum per block): a wave of them takes 1.35 to 1.5 times as long as one of 128 columns
+    // with fast accumulation, 1.6 to 1.67 with slow (4096-cube: 0.92 against 1.20 ms, 1.21 against 1.31 ms), so they pay
+    // unless half as many tiles leave much of a wave idle
     const long long wide = (long long)w.tiles_m * ((w.tiles_n + 1) / 2);
-    p.wide_tiles = p.umma && slices == 1 && p.fast && one_sum &&
-                   (double)((wide + sms - 1) / sms) * 1.75 < (double)((tiles + sms - 1) / sms);
+    p.wide_tiles = p.umma && slices == 1 && one_sum &&
+                   (double)((wide + sms - 1) / sms) * (p.fast ? 1.45 : 1.65) < (double)((tiles + sms - 1) / sms);
     if (slices >= 2) {
       w = wx;
       p.slices = slices;

@@ -43,10 +43,11 @@ struct UmmaTile {
 static_assert(sizeof(UmmaTile) == 16384, "tile layout");
 template <int NW>
 struct UmmaStage { UmmaTile a, b[NW / 64]; };
-template <int NW>
-struct SmemUmma {                              // NW columns per half: 64 (5 stages of 32 KB) or 128 (4 stages of 48 KB)
-  static constexpr int RING = NW == 64 ? 5 : 4;
-  UmmaStage<NW> stage[RING];                   // later: the images of the output tile
+template <int NW, bool PARTS>
+struct SmemUmma {                              // NW columns per half: 64 (5 stages of 32 KB) or 128 (4 stages of 48 KB; 2 with sums)
+  static constexpr int RING = NW == 64 ? 5 : (PARTS ? 2 : 4);
+  UmmaStage<NW> stage[RING];                   // later: the image of the output tile (of one half of it)
+  float part[PARTS ? 2 * NW : 1][128];         // running sums of slow accumulation, [column][row], where TMEM is full
   unsigned long long full[RING];               // the stage's copies have landed
   unsigned long long empty[RING];              // the MMAs that read the stage are done
   unsigned long long ready[2];                 // half h: every warp has stored R of the block (and read its exponent sums)
@@ -134,7 +135,8 @@ __global__ void __launch_bounds__(THREADS) predecode_umma_kernel(const __grid_co
 
 template <int NFMA, int FA, int FB, bool SLOW, int NW, bool SLICED>
 __global__ void __launch_bounds__(UMMA_THREADS, 1) umma_kernel(const __grid_constant__ Params p) {
-  using Smem = SmemUmma<NW>;
+  constexpr bool PARTS = SLOW && !SLICED && NW == 128; // running sums in shared memory
+  using Smem = SmemUmma<NW, PARTS>;
   constexpr bool POW256 = tc_pow_mul(FA, FB) == 8;
   constexpr int RING = Smem::RING, WC = NW / 2;        // columns of a warp
   constexpr int BPT = KT / NFMA;                       // blocks per k-tile
@@ -144,7 +146,6 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) umma_kernel(const __grid_cons
   constexpr int COL_S = 2 * NW;
   constexpr int COL_PART = 384;                        // running sums of chain results (slow accumulation, NW = 64)
   constexpr int CHUNK = TWO_SUMS ? 8 : 16;             // columns a warp handles at a time; the next ones are being loaded
-  static_assert(NW == 64 || !SLOW, "TMEM holds no running sums for 256 columns");
   static_assert(NW == 64 || !TWO_SUMS, "TMEM holds one set of sums for 256 columns");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
@@ -260,7 +261,10 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) umma_kernel(const __grid_cons
 #pragma unroll
     for (int q = 0; q < CHUNK; ++q) zero[q] = R_ZERO;
     for (int c = 0; c < WC; c += CHUNK) tmem_st(my + c, zero);
-    if (SLOW && !SLICED) {
+    float* sums = &sm.part[PARTS ? WC * (warp / 4) : 0][32 * (warp % 4) + lane];
+    if (PARTS) {
+      for (int c = 0; c < WC; ++c) sums[c * 128] = 0.0f;
+    } else if (SLOW && !SLICED) {
       const uint32_t none[CHUNK] = {};
       for (int c = 0; c < WC; c += CHUNK) tmem_st(my + c + COL_PART, none);
     }
@@ -282,17 +286,18 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) umma_kernel(const __grid_cons
         for (int c = 0; c < WC; c += CHUNK) {
           uint32_t r[CHUNK], part[CHUNK];
           tmem_ld(r, my + c);
-          if constexpr (!SLICED) tmem_ld(part, my + c + COL_PART);
+          if constexpr (!SLICED && !PARTS) tmem_ld(part, my + c + COL_PART);
           tmem_wait_ld();
           tmem_use(r);
-          if constexpr (!SLICED) tmem_use(part);
+          if constexpr (!SLICED && !PARTS) tmem_use(part);
 #pragma unroll
           for (int q = 0; q < CHUNK; ++q) {
             const float v = chain_result4(fm::mma_end(__uint_as_float(r[q])));
             if constexpr (SLICED) dst[(size_t)(c + q) * BM] = v;
+            else if constexpr (PARTS) sums[(c + q) * 128] = __fadd_rn(sums[(c + q) * 128], v);
             else part[q] = __float_as_uint(__fadd_rn(__uint_as_float(part[q]), v));
           }
-          if constexpr (!SLICED) tmem_st(my + c + COL_PART, part);
+          if constexpr (!SLICED && !PARTS) tmem_st(my + c + COL_PART, part);
           tmem_st(my + c, zero);
         }
         tmem_wait_st();
@@ -337,35 +342,49 @@ __global__ void __launch_bounds__(UMMA_THREADS, 1) umma_kernel(const __grid_cons
   if (!SLICED && !bad && warp < EPI_WARPS) {           // a K slice has stored its chains; the combine kernel writes the output
     Epilogue epi;
     epi.init(p);
-    // images of 128 x 128 outputs: one, or one per half
-    constexpr int IMAGES = NW / 64, IMAGE_THREADS = EPI_THREADS / IMAGES;
-    unsigned char* image = smem_raw + (IMAGES == 2 ? h * (128 * (128 * 4 + 16)) : 0);
-    const int lr = 32 * (warp % 4) + lane, gm = m0 + lr, nc = n0 + (IMAGES == 2 ? 128 * h : 0);
+    const int lr = 32 * (warp % 4) + lane, gm = m0 + lr;
     const int row_flag = p.patch_nonfinite && gm < p.M ? p.ws_flag_a[gm] : 0;
-    if (h < H) {
+    // an image of 128 x 128 outputs for both halves (NW = 64) or for one after the other; rows of it are written out by all
+    // the warps. Elements beyond M or N are parked too and not written out.
 #pragma unroll 1
-      for (int c = 0; c < WC; c += CHUNK) {
-        uint32_t r[CHUNK];
-        tmem_ld(r, my + c + (SLOW ? COL_PART : 0));
-        tmem_wait_ld();
-        tmem_use(r);
+    for (int half = 0; half < NW / 64; ++half) {
+      const int nc = n0 + 128 * half;
+      if (nc >= p.N) break;
+      if (h < H && (NW == 64 || h == half)) {
+#pragma unroll 1
+        for (int c = 0; c < WC; c += CHUNK) {
+          uint32_t r[CHUNK];
+          float v[CHUNK];
+          const int lc = (WC * (warp / 4) + c) % 128, gn = nc + lc;
+          if constexpr (PARTS) {
 #pragma unroll
-        for (int q = 0; q < CHUNK; ++q) {
-          const int lc = (WC * (warp / 4) + c + q) % 128, gn = nc + lc;
-          float v = __uint_as_float(r[q]);
-          if (!SLOW) v = chain_result4(fm::mma_end(v));
-          if (gm < p.M && gn < p.N) {
-            const int flag = p.patch_nonfinite ? row_flag | p.ws_flag_b[gn] : 0;
-            uint32_t bits;
-            if (flag && nonfinite_patch(flag, p.A + (long long)gm * p.lda, p.B + (long long)gn * p.ldb, p.K, p.fmt_a, p.fmt_b, bits))
-              v = __uint_as_float(bits);
-            epi.park(image, lr, lc, v);
+            for (int q = 0; q < CHUNK; ++q) v[q] = sm.part[WC * (warp / 4) + c + q][lr];
+          } else {
+            tmem_ld(r, my + c + (SLOW ? COL_PART : 0));
+            tmem_wait_ld();
+            tmem_use(r);
+#pragma unroll
+            for (int q = 0; q < CHUNK; ++q) v[q] = SLOW ? __uint_as_float(r[q]) : chain_result4(fm::mma_end(__uint_as_float(r[q])));
           }
+          // non-finite classes: one look for the warp's rows and these columns, then element by element where one is set
+          const int col = gn + lane % CHUNK, col_flag = p.patch_nonfinite && col < p.N ? p.ws_flag_b[col] : 0;
+          if (__any_sync(0xFFFFFFFFu, row_flag | col_flag)) {
+#pragma unroll
+            for (int q = 0; q < CHUNK; ++q) {
+              const int flag = row_flag | __shfl_sync(0xFFFFFFFFu, col_flag, q);
+              uint32_t bits;
+              if (flag && gm < p.M && gn + q < p.N &&
+                  nonfinite_patch(flag, p.A + (long long)gm * p.lda, p.B + (long long)(gn + q) * p.ldb, p.K, p.fmt_a, p.fmt_b, bits))
+                v[q] = __uint_as_float(bits);
+            }
+          }
+          epi.park_row(smem_raw, lr, lc, v);
         }
       }
+      asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
+      epi.flush(p, smem_raw, m0, nc, tid, EPI_THREADS);
+      if (NW == 128) asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
     }
-    asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
-    if (h < H) epi.flush(p, image, m0, nc, tid % IMAGE_THREADS, H == 1 && IMAGES == 1 ? IMAGE_THREADS / 2 : IMAGE_THREADS);
   }
   fence_before();
   __syncthreads();
@@ -386,10 +405,12 @@ cudaError_t launch_predecode(const Params& p, cudaStream_t stream, int* launches
 template <int NFMA, int FA, int FB, bool SLOW, int NW, bool SLICED>
 cudaError_t launch_kernel(const Params& p, cudaStream_t stream, int* launches) {
   auto kern = umma_kernel<NFMA, FA, FB, SLOW, NW, SLICED>;
-  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemUmma<NW>));
+  constexpr size_t SMEM = sizeof(SmemUmma<NW, SLOW && !SLICED && NW == 128>);
+  static_assert(SMEM <= 232448, "shared memory of a CTA");
+  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
   if (err != cudaSuccess) return err;
   const long long tiles = (long long)p.tiles_m * ((p.N + 2 * NW - 1) / (2 * NW));
-  kern<<<dim3((unsigned)tiles, SLICED ? (unsigned)p.slices : 1u), UMMA_THREADS, sizeof(SmemUmma<NW>), stream>>>(p);
+  kern<<<dim3((unsigned)tiles, SLICED ? (unsigned)p.slices : 1u), UMMA_THREADS, SMEM, stream>>>(p);
   err = cudaGetLastError();
   if (err == cudaSuccess) *launches += 1;
   return err;
@@ -401,7 +422,9 @@ cudaError_t launch_main(const Params& p, cudaStream_t stream, int* launches) {
     return p.plan_group ? launch_kernel<NFMA, FA, FB, true, 64, true>(p, stream, launches)
                         : launch_kernel<NFMA, FA, FB, false, 64, true>(p, stream, launches);
   if constexpr (tc_pow_mul(FA, FB) == 8 || NFMA == 16) {
-    if (p.wide_tiles) return launch_kernel<NFMA, FA, FB, false, 128, false>(p, stream, launches);
+    if (p.wide_tiles)
+      return p.fast ? launch_kernel<NFMA, FA, FB, false, 128, false>(p, stream, launches)
+                    : launch_kernel<NFMA, FA, FB, true, 128, false>(p, stream, launches);
   }
   return p.fast ? launch_kernel<NFMA, FA, FB, false, 64, false>(p, stream, launches)
                 : launch_kernel<NFMA, FA, FB, true, 64, false>(p, stream, launches);
