@@ -50,14 +50,12 @@ STRONG = dict(name="cfg5_recipe_16384x16384x8192", profile="hopper", M=16384, N=
 # Executed warp-instruction lanes per emulated multiply-accumulate, from ncu captures of the kernels as committed
 # (smsp__inst_executed.sum * 32 / (M*N*K), profiles/): keyed by (kernel, products per block, accumulation). A workload
 # whose kernel has no capture gets no issue-slot roofline (null), never another kernel's constant.
-INST_PER_MAC = {("staged_tc_kernel", 32, "slow"): 2.514,       # 4096 cube, profiles/staged_tc_kernel_hopper_e4m3_2048cube.md
+INST_PER_MAC = {("umma_kernel", 32, "slow"): 0.345,             # 2048 cube, profiles/umma_kernel_hopper_e4m3_2048cube.md
                 ("staged_kernel", 32, "slow"): 3.16,           # 2048 cube e5m2 x e4m3 with MMAEMU_B200_TC_EPASS=0, profiles/staged_kernel_hopper_e5m2xe4m3_2048cube.md
                 ("fast_kernel", 32, "slow"): 3.37,             # 2048 cube, profiles/fast_kernel_hopper_e4m3_2048cube.md
-                ("staged_kernel, at most 16 rows", 32, "slow"): 5.18,   # 16 x 4096 x 8192, profiles/few_rows_kernel_hopper_e5m2xe4m3_16x4096x8192.md
                 ("integer_kernel", 32, "slow"): 8.56}           # 2048 cube, profiles/integer_kernel_hopper_e4m3_2048cube.md
-# DRAM bytes per launch of the main kernel on the headline workload, one-pass ncu capture at full size
-# (dram__bytes_read.sum + dram__bytes_write.sum = 873,141,504 + 32,601,856; same profile file).
-DRAM_TRAFFIC = {("staged_tc_kernel", 32, "slow", 4096, 4096, 4096): 905743360}
+# DRAM bytes per launch of the main kernel by workload, from one-pass ncu captures at full size: none of the present kernels.
+DRAM_TRAFFIC = {}
 
 
 # ---------------------------------------------------------------------------------------------------------------
@@ -314,11 +312,9 @@ def workload_text(c) -> str:
 
 def kernel_of(cfg, S=1) -> str:
     """Name of the main kernel the automatic choice runs for a configuration (with scratch memory)."""
-    pair = (cfg["fa"], cfg["fb"])
-    name = ("staged_tc_kernel" if pair == ("e4m3", "e4m3") else
-            "staged_kernel" if pair == ("e5m2", "e5m2") else "staged_tc_kernel, powers of 32")
-    # with at most 16 rows (unsplit plans and K slices) the instantiations that decode both operands themselves run
-    return name + ", at most 16 rows" if cfg["M"] <= 16 else name
+    if cfg["M"] <= 16:
+        return "staged_tc_kernel, 16 rows per CTA"
+    return "staged_tc_kernel" if (cfg["fa"], cfg["fb"]) == ("e5m2", "e5m2") else "umma_kernel"
 
 
 class Timer:
@@ -462,7 +458,7 @@ def other_configs(mm, oracle, timer, dev, issue_peak_t):
         off = time_config(mm, oracle, timer, dev, dict(c, name="rowgroups_off"), ra, rb, 0.5, 1.25, 5)
     finally:
         os.environ.pop("MMAEMU_B200_ROW_GROUPS", None)
-    out[c["name"]]["ms_with_8_row_slot_kernels"] = off["ms"]
+    out[c["name"]]["ms_without_row_groups"] = off["ms"]
     out[c["name"]]["kernel"] = "staged_tc_kernel, 16 rows per CTA (row groups)"
     # 4: FP8 projection stack, hopper-te, amax-derived scales
     for i, (N, K) in enumerate([(5760, 1920), (1920, 1920), (24576, 8192)]):
@@ -649,8 +645,8 @@ def run_one_gpu(args) -> int:
         "metric": METRIC, "value": value, "unit": "TFLOP/s", "n_gpus": 1, "steps": args.steps,
         "warmup": max(3, args.warmup), "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None,
-        "dtype": "int32" if used == "integer_kernel" else "fp32 round-toward-zero FMA + int32 (exact emulation of fp8 x "
-                                                         "fp8 blocks)",
+        "dtype": "int32" if used == "integer_kernel" else "fp8 tensor-core products truncated through fp32 offset "
+                                                         "accumulators (exact emulation of fp8 x fp8 blocks)",
         "data": "synthetic",
         "config": {"workload": workload_text(cfg) + f", kernel {used}", "profile": cfg["profile"],
                    "l2": f"flushed between steps ({L2_FLUSH_BYTES >> 20} MiB write)", "multi_gpu": "single GPU"},
