@@ -127,7 +127,8 @@ int mmb200_scaled_mm_host(const void *A_host, int64_t lda, int fmt_a, const void
  * 8.5 per element of B, rounded up to 128 x 32 tiles) and streams the decoded tiles into shared memory with bulk
  * asynchronous copies. mmb200_workspace_bytes gives the size for a shape; the *_ws entry points take the memory from
  * the caller (128-byte aligned, at least that size, used only until the call's work on the stream has finished) and
- * are otherwise identical to mmb200_scaled_mm / mmb200_accumulate. With workspace_dev == NULL, a workspace that is too
+ * are otherwise identical to mmb200_scaled_mm / mmb200_accumulate. 0 means that no scratch-memory kernel takes the shape
+ * (an empty one, or more than 65,535 tiles of 128 rows or columns). With workspace_dev == NULL, a workspace that is too
  * small, or a request the fast kernels do not serve, they behave exactly like the entry points without workspace.
  * The reference has no counterpart: its kernels decode inside the main loop (mmaemu/backends/cuda/csrc/h4.cu:190-211). */
 size_t mmb200_workspace_bytes(int M, int N, int K);

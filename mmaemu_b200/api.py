@@ -316,6 +316,8 @@ def _workspace(L, kernel: str, a_ptr, lda, b_ptr, ldb, M, N, K, nfma, S, device)
     if nfma not in (16, 32):
         return None, None, 0                 # the late-accumulator preset runs on the integer kernel
     n = int(L.mmb200_workspace_bytes_split(M, N, K, S))
+    if n == 0:
+        return None, None, 0                 # more than 65,535 tiles of 128 rows or columns: no staged kernel takes the call
     if S > 1 and n > SPLIT_WORKSPACE_LIMIT:
         return None, None, 0                 # split plans keep 8 bytes of scratch per output; very large ones run on the integer kernel
     ws = torch.empty(n, dtype=torch.uint8, device=device)

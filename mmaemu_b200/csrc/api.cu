@@ -21,7 +21,7 @@ int cuda_fail(cudaError_t err) {
 
 // Status word of a staged launch, read after the stream has drained.
 int read_status(const void* workspace, int M, int N, int K, int S, cudaStream_t st) {
-  if (!workspace || M <= 0 || N <= 0 || K <= 0) return MMB200_OK;
+  if (!workspace || !mmb::staged_workspace_bytes(M, N, K, S, false)) return MMB200_OK;   // nothing waits
   int word = 0;
   cudaError_t err = cudaMemcpyAsync(&word, static_cast<const unsigned char*>(workspace) + mmb::staged_status_offset(M, N, K, S),
                                     sizeof(int), cudaMemcpyDeviceToHost, st);
@@ -384,7 +384,7 @@ int mmb200_scaled_mm_host(const void* A, int64_t lda, int fmt_a, const void* B, 
       tile_rows = ((M + 127) / 128 + PIPELINE_MAX_SLABS - 1) / PIPELINE_MAX_SLABS;
       slabs = ((M + 127) / 128 + tile_rows - 1) / tile_rows;
     }
-    if (slabs >= 2) {
+    if (slabs >= 2 && mmb::staged_workspace_bytes(tile_rows * 128, N, K, S, true, true)) {
       cudaError_t perr = host_pipeline(&pipe);
       if (perr != cudaSuccess) return cuda_fail(perr);
       slab_rows = tile_rows * 128;

@@ -309,9 +309,10 @@ cudaError_t launch_fast(const Params& p, int nfma, cudaStream_t stream);
 // tcgen05 kernels (kernel_umma.cu), called by the staged launches: operand images, then the GEMM; p filled in by them.
 cudaError_t launch_umma(const Params& p, int nfma, cudaStream_t stream, int* launches);
 bool fast_supports(const Params& p, int nfma);
-// Staged fast kernel: scratch bytes it needs for a shape, and the launch (pre-decode of both operands, then the GEMM).
+// Staged fast kernel: scratch bytes it needs for a shape (0: a shape it does not take), and the launch (pre-decode of both
+// operands, then the GEMM).
 // `launches` is increased by the number of kernels launched.
-bool staged_supports(const Params& p, int nfma);            // any plan, any operands (with scratch memory)
+bool staged_supports(const Params& p, int nfma);            // any plan, any operands (with scratch memory), up to 65,535 tiles
 bool staged_vector_supports(const Params& p, int nfma);     // any plan, operands that 16-byte loads can read
 size_t staged_workspace_bytes(int M, int N, int K, int S, bool with_slices, bool shared_b = false);
 // Bytes of a shared B area (tile images of every 128-column group, then one int per column), and the launch that fills

@@ -1266,10 +1266,18 @@ bool vector_loads(const Params& p) {
   return (p.K % 16) == 0 && !((reinterpret_cast<uintptr_t>(p.A) | reinterpret_cast<uintptr_t>(p.B)) & 15) && !((p.lda | p.ldb) & 15);
 }
 }  // namespace
-bool staged_supports(const Params& p, int nfma) {
+namespace {
+// The staged launches put the tiles of an operand into grid y (65,535 at most) and the output tiles into grid x.
+bool staged_grid_ok(int M, int N) {
+  const long long tm = ((long long)M + BM - 1) / BM, tn = ((long long)N + BN - 1) / BN;
+  return tm <= 65535 && tn <= 65535 && tm * tn <= 0x7FFFFFFFLL;
+}
+bool plan_ok(const Params& p, int nfma) {
   return (nfma == 16 || nfma == 32) && p.S >= 1 && p.S <= MMB200_MAX_SPLITS && p.K > 0;
 }
-bool fast_supports(const Params& p, int nfma) { return p.S == 1 && staged_supports(p, nfma) && vector_loads(p); }
+}  // namespace
+bool staged_supports(const Params& p, int nfma) { return plan_ok(p, nfma) && staged_grid_ok(p.M, p.N); }
+bool fast_supports(const Params& p, int nfma) { return p.S == 1 && plan_ok(p, nfma) && vector_loads(p); }
 bool staged_vector_supports(const Params& p, int nfma) { return staged_supports(p, nfma) && vector_loads(p); }
 
 cudaError_t launch_fast(const Params& p_in, int nfma, cudaStream_t stream) {
@@ -1284,7 +1292,7 @@ cudaError_t launch_fast(const Params& p_in, int nfma, cudaStream_t stream) {
 }
 
 size_t staged_workspace_bytes(int M, int N, int K, int S, bool with_slices, bool shared_b) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (M <= 0 || N <= 0 || K <= 0 || !staged_grid_ok(M, N)) return 0;
   return workspace_layout(M, N, K, S < 1 ? 1 : S, with_slices, shared_b).total;
 }
 
@@ -1338,7 +1346,7 @@ cudaError_t launch_staged(const Params& p_in, int nfma, void* workspace, size_t 
   if (shared_b && (reinterpret_cast<uintptr_t>(p.shared_b) & 127)) return cudaErrorInvalidValue;
   WorkspaceLayout w = workspace_layout(p.M, p.N, p.K, p.S, false, shared_b);
   if (!workspace || workspace_bytes < w.total || (reinterpret_cast<uintptr_t>(workspace) & 127)) return cudaErrorInvalidValue;
-  if ((long long)w.tiles_m * w.tiles_n > 0x7FFFFFFFLL || w.tiles_m > 65535 || w.tiles_n > 65535) return cudaErrorInvalidValue;
+  if (!staged_grid_ok(p.M, p.N)) return cudaErrorInvalidValue;
   {
     const char* env = std::getenv("MMAEMU_B200_TC_EPASS");         // "0": the packed-integer exponent pass for every pair
     if (env && env[0] == '0' && env[1] == 0) p.no_tensor_epass = 1;

@@ -71,7 +71,8 @@ extern "C" int mmb200_scaled_mm_static(const void* A, int64_t lda, int fmt_a, co
   if (M == 0 || N == 0) return MMB200_OK;
   // only requests the scratch-memory kernel serves: unsplit plan, K % 16 == 0, 16-byte aligned operands
   if (K == 0 || mmb200_kernel_for(A, lda, B, ldb, K, nfma, 1) != MMB200_KERNEL_FAST) return MMB200_ERR_UNSUPPORTED;
-  if (mmb200_workspace_bytes(M, N, K) > SCRATCH_BYTES) return MMB200_ERR_TOO_LARGE;
+  const size_t need = mmb200_workspace_bytes(M, N, K);
+  if (need == 0 || need > SCRATCH_BYTES) return MMB200_ERR_TOO_LARGE;   // 0: beyond the grid limit of the scratch-memory kernels
   int status = MMB200_OK;
   void* scratch = scratch_on_current_device(&status);
   if (!scratch) return status;

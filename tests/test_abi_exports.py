@@ -65,6 +65,14 @@ def test_status_codes_and_argument_checks_without_a_device(lib):
     assert lib.mmb200_launch_count() == 0
 
 
+def test_shapes_beyond_the_grid_of_the_scratch_memory_kernels_ask_for_no_scratch(lib):
+    """65,535 tiles of 128 rows or columns are the most that one launch takes; the integer kernel serves larger shapes."""
+    most = 65535 * 128
+    for M, N in ((most + 1, 16), (16, most + 1)):
+        assert lib.mmb200_workspace_bytes(M, N, 32) == 0 and lib.mmb200_workspace_bytes_split(M, N, 32, 2) == 0
+    assert lib.mmb200_workspace_bytes(most, 16, 32) > 0 and lib.mmb200_workspace_bytes(16, most, 32) > 0
+
+
 def test_no_device_is_a_status_not_a_crash(lib):
     import torch
     if torch.cuda.is_available():

@@ -191,6 +191,22 @@ def test_accumulate_any_k():
         assert np.array_equal(bits(acc), oracle.accumulate(a, b, fmt_a="e4m3", fmt_b="e5m2", preset="ada", fast=False))
 
 
+@pytest.mark.parametrize("M,N", ((65535 * 128 + 1, 2), (2, 65535 * 128 + 1)))
+def test_accumulate_beyond_the_grid_of_the_scratch_memory_kernels(M, N):
+    """More than 65,535 tiles of 128 rows or columns: such a call runs on the integer kernel. Every row of the long operand is
+    one of 256 kinds, so the oracle computes 256 of them."""
+    rng = np.random.default_rng(3)
+    kinds, other = rng.integers(0, 0x78, (256, 3), dtype=np.uint8), rng.integers(0, 0x78, (2, 3), dtype=np.uint8)
+    long = torch.from_numpy(kinds).to(DEV).repeat(max(M, N) // 256 + 1, 1)[:max(M, N)].contiguous().view(F8["e4m3"])
+    short = torch.from_numpy(other).to(DEV).view(F8["e4m3"])
+    a, b = (long, short) if M > N else (short, long)
+    acc = mm.accumulate(a, b, use_fast_accum=True, profile="hopper", splitk=1)
+    want = oracle.accumulate(kinds, other, preset="hopper", fast=True).view(np.int32)
+    got = (acc if M > N else acc.t()).contiguous().view(torch.int32)
+    want = torch.from_numpy(want.copy()).to(DEV).repeat(max(M, N) // 256 + 1, 1)[:max(M, N)]
+    assert torch.equal(got, want)
+
+
 def test_backend_object_chain_fn():
     from types import SimpleNamespace
     from mmaemu_b200.backend import BACKEND
