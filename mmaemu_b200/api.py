@@ -307,8 +307,9 @@ SPLIT_WORKSPACE_LIMIT = 8 << 30
 
 
 def _workspace(L, kernel: str, a_ptr, lda, b_ptr, ldb, M, N, K, nfma, S, device):
-    """(keep-alive tensor or None, pointer or None, bytes) of the scratch memory for the staged fast kernel. The tensor
-    comes from torch's caching allocator, which hands it out again only to later work on the same stream."""
+    """(keep-alive tensor or None, pointer or None, bytes) of the scratch memory for the staged fast kernel; none where the
+    device has too little memory left for it. The tensor comes from torch's caching allocator, which hands it out again only
+    to later work on the same stream."""
     if kernel in ("integer", "direct") or os.environ.get("MMAEMU_B200_WORKSPACE", "1") == "0":
         return None, None, 0
     if kernel != "auto" and L.mmb200_kernel_for(a_ptr, lda, b_ptr, ldb, K, nfma, 1) != _lib.KERNEL_CODES["fast"]:
@@ -320,7 +321,10 @@ def _workspace(L, kernel: str, a_ptr, lda, b_ptr, ldb, M, N, K, nfma, S, device)
         return None, None, 0                 # more than 65,535 tiles of 128 rows or columns: no staged kernel takes the call
     if S > 1 and n > SPLIT_WORKSPACE_LIMIT:
         return None, None, 0                 # split plans keep 8 bytes of scratch per output; very large ones run on the integer kernel
-    ws = torch.empty(n, dtype=torch.uint8, device=device)
+    try:
+        ws = torch.empty(n, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return None, None, 0                 # the kernels that need no scratch memory serve every call, more slowly
     return ws, ws.data_ptr(), n
 
 

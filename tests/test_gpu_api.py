@@ -207,6 +207,27 @@ def test_accumulate_beyond_the_grid_of_the_scratch_memory_kernels(M, N):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("K", (64, 67))
+def test_a_call_without_memory_left_for_scratch_is_served(K, monkeypatch):
+    """The scratch memory makes a call faster and is not needed to answer it: where it cannot be had, the kernels without it
+    run. The allocation fails here because the test makes it fail; nothing is driven out of memory."""
+    from mmaemu_b200 import api
+    a, b, ta, tb = operands(40, 72, K, seed=11)
+    empty, refused = torch.empty, []
+
+    def without_scratch(*size, dtype=None, **kw):
+        if dtype is torch.uint8:
+            refused.append(size)
+            raise torch.OutOfMemoryError("no memory left")
+        return empty(*size, dtype=dtype, **kw)
+    monkeypatch.setattr(api.torch, "empty", without_scratch)
+    for splitk, fast in ((1, True), ((2, "contiguous"), False)):
+        acc = mm.accumulate(ta, tb, use_fast_accum=fast, profile="hopper", splitk=splitk)
+        S, scheme = (1, "none") if splitk == 1 else splitk
+        assert np.array_equal(bits(acc), oracle.accumulate(a, b, preset="hopper", fast=fast, S=S, scheme=scheme))
+    assert refused
+
+
 def test_backend_object_chain_fn():
     from types import SimpleNamespace
     from mmaemu_b200.backend import BACKEND
