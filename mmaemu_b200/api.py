@@ -328,6 +328,15 @@ def _workspace(L, kernel: str, a_ptr, lda, b_ptr, ldb, M, N, K, nfma, S, device)
     return ws, ws.data_ptr(), n
 
 
+def _check_waits(L, ws, M, N, K, S, dev) -> None:
+    """Opt-in ($MMAEMU_B200_CHECK_STATUS=1): wait for the call that used the scratch memory `ws` and raise if one of its
+    bounded waits ran out (a host synchronisation per call)."""
+    if ws is None or os.environ.get("MMAEMU_B200_CHECK_STATUS", "0") != "1":
+        return
+    with _on_device(dev):
+        _lib.check("mmb200_workspace_status", L.mmb200_workspace_status(ws.data_ptr(), M, N, K, S, _stream_ptr(dev)))
+
+
 def _kernel_code(kernel: str) -> int:
     return _lib.KERNEL_CODES["auto" if kernel == "direct" else kernel]
 
@@ -358,11 +367,7 @@ def _run_scaled_mm(c: _Call, mat2, scale_a, scale_b, scale_result, fast: bool, y
                                       _lib.SCHEME_CODES[c.scheme], pa, pb, pr, _kernel_code(c.kernel), ws_ptr, ws_bytes,
                                       peer_array, len(peers), _stream_ptr(dev))
     _lib.check("mmb200_scaled_mm_peers", rc)
-    if ws is not None and os.environ.get("MMAEMU_B200_CHECK_STATUS", "0") == "1":
-        # opt-in: wait for the call and read the status word of its bounded waits (a host synchronisation per call)
-        with torch.cuda.device(dev):
-            _lib.check("mmb200_workspace_status", L.mmb200_workspace_status(ws_ptr, c.M, c.N, c.K, c.decision.S,
-                                                                            _stream_ptr(dev)))
+    _check_waits(L, ws, c.M, c.N, c.K, c.decision.S, dev)
     del keep_a, keep_b, keep_r, ws
     return y
 
@@ -541,6 +546,7 @@ def quantized_scaled_mm(x, quant_scale, mat2, scale_a, scale_b, scale_result=Non
                                             int(bool(use_fast_accum)), c.decision.S, _lib.SCHEME_CODES[c.scheme], pa, pb,
                                             pr, ws.data_ptr(), n, _stream_ptr(dev))
     _lib.check("mmb200_quantize_scaled_mm_ws", rc)
+    _check_waits(L, ws, c.M, c.N, c.K, c.decision.S, dev)
     del keep_q, keep_a, keep_b, keep_r, ws
     return (y, xq) if return_codes else y
 
@@ -589,6 +595,7 @@ def accumulate(a, b, *, use_fast_accum, profile=None, splitk="auto", backend="au
                                     acc.data_ptr(), N, M, N, K, preset.code, int(fast), decision.S,
                                     _lib.SCHEME_CODES[scheme], _kernel_code(kernel), ws_ptr, ws_bytes, _stream_ptr(dev))
     _lib.check("mmb200_accumulate_ws", rc)
+    _check_waits(L, ws, M, N, K, decision.S, dev)
     del ws
     return acc
 

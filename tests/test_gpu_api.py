@@ -407,6 +407,13 @@ def test_a_wait_that_runs_out_is_reported_and_nothing_is_written(monkeypatch):
         with pytest.raises(_lib.NativeError):
             mm.scaled_mm(a.view(torch.float8_e4m3fn), b.view(torch.float8_e4m3fn).t(), sc[0], sc[1],
                          out_dtype=torch.bfloat16, use_fast_accum=True, profile="hopper", splitk=1)
+        for k in (K, K - 3):                                       # and the other two, odd K included
+            with pytest.raises(_lib.NativeError):
+                mm.accumulate(a[:, :k].view(torch.float8_e4m3fn), b[:, :k].view(torch.float8_e4m3fn), use_fast_accum=True,
+                              profile="hopper", splitk=1)
+        with pytest.raises(_lib.NativeError):
+            mm.quantized_scaled_mm(torch.ones(M, K, device=DEV), sc[1], b.view(torch.float8_e4m3fn).t(), sc[0], sc[1],
+                                   out_dtype=torch.bfloat16, use_fast_accum=True, profile="hopper", splitk=1)
     finally:
         os.environ.pop("MMAEMU_B200_CHECK_STATUS", None)
         L.mmb200_test_hooks(0, 0)
