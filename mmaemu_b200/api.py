@@ -32,7 +32,7 @@ from . import _lib
 from .errors import (BackendUnavailableError, ExperimentalPresetWarning, ReferenceRejectsError,
                      UnsupportedFeatureError)
 from .formats import E4M3, E5M2, OUT_DTYPE_NAMES, fmt_of, is_fp8_dtype
-from .numerics import check_plan, get_preset, maturity_warning, warn_once
+from .numerics import check_plan, get_preset, has_empty_splits, maturity_warning, warn_once
 from .platforms import get_profile, profile_maturity_warning
 from .splitk import resolve_splitk
 
@@ -306,13 +306,14 @@ def _on_device(dev):
 SPLIT_WORKSPACE_LIMIT = 8 << 30
 
 
-def _workspace(L, kernel: str, a_ptr, lda, b_ptr, ldb, M, N, K, nfma, S, device):
+def _workspace(L, kernel: str, a_ptr, lda, b_ptr, ldb, M, N, K, nfma, S, scheme, device):
     """(keep-alive tensor or None, pointer or None, bytes) of the scratch memory for the staged fast kernel; none where the
     device has too little memory left for it. The tensor comes from torch's caching allocator, which hands it out again only
     to later work on the same stream."""
     if kernel in ("integer", "direct") or os.environ.get("MMAEMU_B200_WORKSPACE", "1") == "0":
         return None, None, 0
-    if kernel != "auto" and L.mmb200_kernel_for(a_ptr, lda, b_ptr, ldb, K, nfma, 1) != _lib.KERNEL_CODES["fast"]:
+    if (kernel != "auto" or has_empty_splits(K, S, scheme)) and \
+            L.mmb200_kernel_for(a_ptr, lda, b_ptr, ldb, K, nfma, 1) != _lib.KERNEL_CODES["fast"]:
         return None, None, 0                 # operands the fast kernels cannot read with 16-byte loads
     if nfma not in (16, 32):
         return None, None, 0                 # the late-accumulator preset runs on the integer kernel
@@ -360,7 +361,7 @@ def _run_scaled_mm(c: _Call, mat2, scale_a, scale_b, scale_result, fast: bool, y
     peer_array = (ctypes.c_void_p * len(peers))(*[ctypes.c_void_p(int(p)) for p in peers]) if peers else None
     with _on_device(dev):
         ws, ws_ptr, ws_bytes = _workspace(L, c.kernel, a.data_ptr(), lda, bt.data_ptr(), ldb, c.M, c.N, c.K,
-                                          c.preset.code, c.decision.S, dev)
+                                          c.preset.code, c.decision.S, c.scheme, dev)
         rc = L.mmb200_scaled_mm_peers(a.data_ptr(), lda, _lib.FMT_CODES[c.fa], bt.data_ptr(), ldb,
                                       _lib.FMT_CODES[c.fb], y.data_ptr(), ldd, _lib.OUT_CODES[OUT_DTYPE_NAMES[c.od]],
                                       c.M, c.N, c.K, c.preset.code, int(fast), c.decision.S,
@@ -590,7 +591,7 @@ def accumulate(a, b, *, use_fast_accum, profile=None, splitk="auto", backend="au
     L = _lib.load()
     with torch.cuda.device(dev):
         ws, ws_ptr, ws_bytes = _workspace(L, kernel, au.data_ptr(), K, bu.data_ptr(), K, M, N, K, preset.code,
-                                          decision.S, dev)
+                                          decision.S, scheme, dev)
         rc = L.mmb200_accumulate_ws(au.data_ptr(), K, _lib.FMT_CODES[fa], bu.data_ptr(), K, _lib.FMT_CODES[fb],
                                     acc.data_ptr(), N, M, N, K, preset.code, int(fast), decision.S,
                                     _lib.SCHEME_CODES[scheme], _kernel_code(kernel), ws_ptr, ws_bytes, _stream_ptr(dev))

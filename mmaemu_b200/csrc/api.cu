@@ -106,9 +106,11 @@ int run(const void* A, int64_t lda, int fmt_a, const void* B, int64_t ldb, int f
   // fast kernels: every plan with enough scratch memory (staged), unsplit plans without; else the integer kernel
   const bool direct_ok = mmb::fast_supports(p, nfma);
   // A request for the fast kernels by name, the quantise prologue and a shared B area keep to operands that 16-byte loads
-  // can read; the automatic choice takes any operand to the staged kernels (1003 x 2001 operands with 517 rows: 592 us on
-  // the integer kernel before)
-  const bool any_operand = kernel == MMB200_KERNEL_AUTO && !a_hp && !shared_b;
+  // can read; the automatic choice takes any operand to the staged kernels (517 x 1003 x 2001: 75 us of kernels, 592 us on the
+  // integer kernel) -- but not plans with empty splits, which their walker visits one by one at several us each (300 x 300 x 33
+  // split in five: 84 us, 45 us on the integer kernel).
+  const bool any_operand = kernel == MMB200_KERNEL_AUTO && !a_hp && !shared_b &&
+                           !(S > 1 && mmb::plan_has_empty_splits(mmb::make_plan(K, p.fast, S, p.scheme)));
   const bool staged_ok = (any_operand ? mmb::staged_supports(p, nfma) : mmb::staged_vector_supports(p, nfma)) && workspace &&
                          workspace_bytes >= mmb::staged_workspace_bytes(M, N, K, S, false, shared_b != nullptr) &&
                          !(reinterpret_cast<uintptr_t>(workspace) & 127);

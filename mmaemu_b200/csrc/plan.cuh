@@ -66,6 +66,11 @@ MMB_PLAN_HD void split_tiles(const Plan& p, int s, int& first, int& end, int& st
   }
 }
 
+// Whether a split owns no tiles (its partial is +0).
+MMB_PLAN_HD bool plan_has_empty_splits(const Plan& p) {
+  return p.contiguous ? (long long)(p.S - 1) * p.q >= p.T : p.S > p.T;
+}
+
 // Order in which the split partials are consumed: serial 0, 1, ..., S-1; pairwise S-1, 0, h, 1, h+1, ... with
 // h = ceil(S / 2) (slot_i = p_i + p_(i+h) if i + h < S - 1 else p_i; result ((p_(S-1) + slot_0) + slot_1) ...).
 // `role` tells the combiner what to do with the partial: 0 = start the total, 1 = start a slot, 2 = add to the slot

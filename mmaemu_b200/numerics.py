@@ -136,3 +136,11 @@ def check_plan(preset: Preset, K: int, S: int, scheme: str, fast: bool = True) -
         raise ValueError(f"scheme {scheme!r} is not a split-K layout of preset {preset.name!r}: its cuBLASLt kernels "
                          f"split as {allowed}")
     return scheme
+
+
+def has_empty_splits(K: int, S: int, scheme: str) -> bool:
+    """Whether a plan that check_plan accepted has a split without k-tiles (plan_has_empty_splits of csrc/plan.cuh)."""
+    if S == 1:
+        return False
+    T = -(-K // (128 if scheme == "contiguous" else 64))
+    return (S - 1) * -(-T // S) >= T if scheme == "contiguous" else S > T

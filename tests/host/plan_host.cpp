@@ -32,3 +32,7 @@ extern "C" int plan_sequence_lanes_host(int K, int fast, int S, int scheme, uint
     if (mmb::plan_sequence(plan, K, out, lane, lanes) != n) return 0;
   return n;
 }
+
+extern "C" int plan_has_empty_splits_host(int K, int fast, int S, int scheme) {
+  return mmb::plan_has_empty_splits(mmb::make_plan(K, fast, S, scheme)) ? 1 : 0;
+}

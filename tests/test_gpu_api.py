@@ -276,6 +276,18 @@ def test_launch_accounting(monkeypatch):
         assert _lib.launch_count() == n0 + 7          # a split plan in K slices: tile order, K slices, combine
 
 
+@pytest.mark.parametrize("profile,splitk,K", (("hopper", (3, "contiguous"), 65), ("ada", (5, "pairwise"), 33), ("ada", (2, "serial"), 63)))
+def test_unaligned_plans_with_empty_splits_run_on_the_integer_kernel(profile, splitk, K):
+    a, b, ta, tb = operands(70, 90, K, "e5m2", "e4m3", seed=K)
+    n0 = _lib.launch_count()
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        acc = mm.accumulate(ta, tb, use_fast_accum=False, profile=profile, splitk=splitk)
+    assert _lib.launch_count() == n0 + 1
+    want = oracle.accumulate(a, b, fmt_a="e5m2", fmt_b="e4m3", preset=profile, fast=False, S=splitk[0], scheme=splitk[1])
+    assert np.array_equal(bits(acc), want)
+
+
 def test_call_is_capturable_in_a_cuda_graph():
     """No host synchronisation anywhere in the call (scales and non-finite flags stay on the device), so a scaled_mm
     call can be captured once and replayed on new operand values -- the gap the reference documents for its CUDA path

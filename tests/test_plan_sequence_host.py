@@ -146,3 +146,14 @@ def test_workers_write_the_same_sequence(lib, fast):
 def test_capacity_is_reported(lib):
     buf = np.zeros(4, np.uint32)
     assert lib.plan_sequence_host(4096, 1, 3, SCHEME["contiguous"], buf.ctypes.data, 4) == -128
+
+
+def test_empty_splits(lib):
+    """The library's and the package's answer to "has a split no k-tiles?" against the sequence itself."""
+    from mmaemu_b200.numerics import has_empty_splits
+    lib.plan_has_empty_splits_host.argtypes = [ctypes.c_int] * 4
+    for S, scheme in [(1, "none")] + CASES + [(64, "serial"), (64, "contiguous")]:
+        for K in (1, 63, 64, 65, 128, 129, 208, 257, 1024, 1936, 4097, 8192):
+            want = any(int(e) & EMPTY for e in sequence(lib, K, True, S, scheme))
+            assert has_empty_splits(K, S, scheme) == want, (K, S, scheme)
+            assert bool(lib.plan_has_empty_splits_host(K, 1, S, SCHEME[scheme])) == want, (K, S, scheme)
