@@ -1388,12 +1388,17 @@ cudaError_t launch_staged(const Params& p_in, int nfma, void* workspace, size_t 
     // Kernel choice by estimated time, in microseconds per k-tile of 32 and wave of CTAs (measured on whole calls at K = 4096,
     // overheads taken off): a 16-row CTA, alone on an SM or two sharing it; a 128 x 128 tile on tcgen05 (16 / 32 products
     // per block) or on mma.sync; 256 columns per tcgen05 CTA. K slices add two launches (SLICE_LAUNCH) and, per chain, the
-    // traffic of the chain results.
+    // traffic of the chain results. On the CUDA cores (MMAEMU_B200_TC_EPASS=0) a 16-row CTA takes 0.26 of a tile's time, two on
+    // an SM 0.364, and the launches are small beside both (256-cube, slow: 22.7 us in two slices, 32.9 in one pass; 1024-cube,
+    // fast, 16 products: 298 us on 16-row CTAs, 392 on tiles).
     const long long sms = sm_count();
     const bool umma_any = umma_supports(p) && !(shared_b && p.S > 1), umma_whole = umma_any && p.S == 1;
-    const double ROWS16 = nfma == 32 ? 0.95 : 1.25, ROWS16_PAIR = nfma == 32 ? 1.35 : 1.75, SLICE_LAUNCH = 8.0;
+    const bool alu = p.no_tensor_epass != 0;
     const bool one_sum = nfma == 16 || (p.fmt_a == MMB200_FMT_E4M3 && p.fmt_b == MMB200_FMT_E4M3);
-    const double UMMA = nfma == 16 ? 2.2 : (one_sum ? 1.3 : 1.65), MMA = nfma == 16 ? 3.3 : 3.0, PREDECODE = 12.0;
+    const double UMMA = nfma == 16 ? 2.2 : (one_sum ? 1.3 : 1.65), MMA = alu ? 8.0 : (nfma == 16 ? 3.3 : 3.0);
+    const double ROWS16 = alu ? 0.26 * MMA : (nfma == 32 ? 0.95 : 1.25);
+    const double ROWS16_PAIR = alu ? 0.364 * MMA : (nfma == 32 ? 1.35 : 1.75);
+    const double SLICE_LAUNCH = alu ? 0.0 : 8.0, PREDECODE = alu ? 0.0 : 12.0, MARGIN = alu ? 0.9 : 0.95;
     auto waves16 = [&](long long n) {
       const long long pairs = n / (2 * sms), rest = n % (2 * sms);
       return pairs * ROWS16_PAIR + (rest == 0 ? 0.0 : (rest <= sms ? ROWS16 : ROWS16_PAIR));
@@ -1412,7 +1417,7 @@ cudaError_t launch_staged(const Params& p_in, int nfma, void* workspace, size_t 
       // a short unsplit problem is done before the launches of a second pass would be
       if (p.S == 1 && s16 > 1 && sliced(waves16(tiles16), 1) < sliced(waves16(tiles16 * s16), s16)) s16 = 1;
       const double time16 = sliced(waves16(tiles16 * s16), s16);
-      if (rows16 || ((p.S == 1 || s16 >= 2) && time16 < 0.95 * time128)) {
+      if (rows16 || ((p.S == 1 || s16 >= 2) && time16 < MARGIN * time128)) {
         slices = rows16 && p.S > 1 && s16 < 2 ? s128 : s16;
         p.row_groups = rows16 ? 1 : 8;
         rows16 = true;

@@ -288,6 +288,19 @@ def test_unaligned_plans_with_empty_splits_run_on_the_integer_kernel(profile, sp
     assert np.array_equal(bits(acc), want)
 
 
+@pytest.mark.parametrize("profile,n,fast,launches", (("hopper", 256, False, 3), ("ada", 1024, True, 1)))
+def test_kernel_choice_on_the_cuda_cores(profile, n, fast, launches, monkeypatch):
+    """MMAEMU_B200_TC_EPASS=0: the choice goes by the CUDA-core kernels' times. The 256-cube runs in two K slices (tile order,
+    slices, combine), the 1024-cube on 16-row CTAs, which need no pre-decode launches."""
+    a, b, ta, tb = operands(n, n, n, seed=n)
+    monkeypatch.setenv("MMAEMU_B200_TC_EPASS", "0")
+    n0 = _lib.launch_count()
+    acc = mm.accumulate(ta, tb, use_fast_accum=fast, profile=profile, splitk=1)
+    assert _lib.launch_count() == n0 + launches
+    rows = slice(0, n, 97)
+    assert np.array_equal(bits(acc)[rows], oracle.accumulate(a[rows], b, preset=profile, fast=fast))
+
+
 def test_call_is_capturable_in_a_cuda_graph():
     """No host synchronisation anywhere in the call (scales and non-finite flags stay on the device), so a scaled_mm
     call can be captured once and replayed on new operand values -- the gap the reference documents for its CUDA path
