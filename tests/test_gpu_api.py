@@ -301,6 +301,21 @@ def test_kernel_choice_on_the_cuda_cores(profile, n, fast, launches, monkeypatch
     assert np.array_equal(bits(acc)[rows], oracle.accumulate(a[rows], b, preset=profile, fast=fast))
 
 
+def test_no_device_switch_on_the_current_device(monkeypatch):
+    """A call on the device that is current does not switch to it (3 us of host time, more than a tenth of a tiny call)."""
+    a, b, ta, tb = operands(17, 17, 17, seed=5)
+    s = torch.ones(1, device=DEV)
+
+    class Switch(torch.cuda.device):
+        def __enter__(self):
+            raise AssertionError("device switch")
+    monkeypatch.setattr(torch.cuda, "device", Switch)
+    acc = mm.accumulate(ta, tb, use_fast_accum=False, profile="hopper", splitk=1)
+    ta, tb = ta[:16, :16].contiguous(), tb[:16, :16].contiguous()
+    mm.scaled_mm(ta, tb.t(), s, s, out_dtype=torch.bfloat16, profile="hopper", splitk=1)
+    assert np.array_equal(bits(acc), oracle.accumulate(a, b, preset="hopper", fast=False))
+
+
 def test_call_is_capturable_in_a_cuda_graph():
     """No host synchronisation anywhere in the call (scales and non-finite flags stay on the device), so a scaled_mm
     call can be captured once and replayed on new operand values -- the gap the reference documents for its CUDA path
