@@ -11,19 +11,29 @@ query on the profile's own GPU" step does not exist here (matches_device is alwa
 """
 from __future__ import annotations
 
-import os
 import functools
+import os
 from dataclasses import dataclass
 
 DEFAULT_PROFILE = "hopper"
 
 
-@functools.lru_cache(maxsize=64)
-def _dtype_name(dt):
-    if dt is None:
-        return None
+def _plain_name(dt):
     s = str(dt)
     return s[6:] if s.startswith("torch.") else s
+
+
+_cached_name = functools.lru_cache(maxsize=64)(_plain_name)
+
+
+def _dtype_name(dt):
+    """The dtype's name without "torch."; cached for hashable arguments (every call asks for several)."""
+    if dt is None:
+        return None
+    try:
+        return _cached_name(dt)
+    except TypeError:                                    # unhashable: no dtype, but an answer all the same
+        return _plain_name(dt)
 
 
 _FMT_ALIASES = {"float8_e4m3fn": "e4m3", "float8_e5m2": "e5m2"}

@@ -166,6 +166,11 @@ def test_profiles_and_env(monkeypatch):
         mm.scaled_mm(a, bt, s, s, out_dtype=torch.bfloat16, profile="ada")
 
 
+def test_rejection_of_arguments_that_are_no_dtypes():
+    assert mm.get_profile("hopper").rejection(["e4m3"], "e4m3", "float8_e5m2") is None
+    assert mm.get_profile("hopper").rejection("e4m3", E4, torch.float8_e5m2) is not None
+
+
 def test_accumulate_argument_checks():
     a, b = torch.zeros(4, 16).to(E4), torch.zeros(5, 16).to(E4)
     with pytest.raises(TypeError):
