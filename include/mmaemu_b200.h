@@ -123,8 +123,8 @@ int mmb200_scaled_mm_host(const void *A_host, int64_t lda, int fmt_a, const void
                           int scheme, float scale_a, float scale_b, const float *scale_result /* host, nullable */,
                           int kernel, void *stream);
 
-/* Scratch memory. The fastest path decodes both operands once into device scratch memory (10 bytes per element of A,
- * 8.5 per element of B, rounded up to 128 x 32 tiles) and streams the decoded tiles into shared memory with bulk
+/* Scratch memory. The fastest path decodes both operands once into device scratch memory (4 bytes per element, rounded up
+ * to 128 x 32 tiles; 10 per element of A and 8 of B while $MMAEMU_B200_TC_EPASS is 0) and streams the decoded tiles into shared memory with bulk
  * asynchronous copies. mmb200_workspace_bytes gives the size for a shape; the *_ws entry points take the memory from
  * the caller (128-byte aligned, at least that size, used only until the call's work on the stream has finished) and
  * are otherwise identical to mmb200_scaled_mm / mmb200_accumulate. 0 means that no scratch-memory kernel takes the shape

@@ -21,9 +21,9 @@ int cuda_fail(cudaError_t err) {
 
 // Status word of a staged launch, read after the stream has drained.
 int read_status(const void* workspace, int M, int N, int K, int S, cudaStream_t st) {
-  if (!workspace || !mmb::staged_workspace_bytes(M, N, K, S, false)) return MMB200_OK;   // nothing waits
+  if (!workspace || !mmb::staged_workspace_bytes(M, N, K, S, false, false, false)) return MMB200_OK;   // nothing waits
   int word = 0;
-  cudaError_t err = cudaMemcpyAsync(&word, static_cast<const unsigned char*>(workspace) + mmb::staged_status_offset(M, N, K, S),
+  cudaError_t err = cudaMemcpyAsync(&word, static_cast<const unsigned char*>(workspace) + mmb::staged_status_offset(M, N),
                                     sizeof(int), cudaMemcpyDeviceToHost, st);
   if (err == cudaSuccess) err = cudaStreamSynchronize(st);
   if (err != cudaSuccess) return cuda_fail(err);
@@ -45,7 +45,7 @@ int run(const void* A, int64_t lda, int fmt_a, const void* B, int64_t ldb, int f
         const float* sr, int epilogue, int patch, int kernel, void* stream, void* workspace = nullptr,
         size_t workspace_bytes = 0, const void* a_hp = nullptr, int64_t ld_hp = 0, int hp_dtype = 0,
         const float* quant_scale = nullptr, void* const* peer_D = nullptr, int n_peers = 0,
-        unsigned char* shared_b = nullptr) {
+        unsigned char* shared_b = nullptr, bool alu = mmb::tensor_cores_off()) {
   if (n_peers < 0 || n_peers > MMB200_MAX_PEERS || (n_peers > 0 && !peer_D)) return MMB200_ERR_BAD_ARG;
   for (int q = 0; q < n_peers; ++q)
     if (!peer_D[q]) return MMB200_ERR_BAD_ARG;
@@ -90,6 +90,7 @@ int run(const void* A, int64_t lda, int fmt_a, const void* B, int64_t ldb, int f
   p.n_peers = n_peers;
   for (int q = 0; q < n_peers; ++q) p.peer_D[q] = peer_D[q];
   p.shared_b = shared_b;
+  p.no_tensor_epass = alu ? 1 : 0;
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t err;
@@ -112,7 +113,7 @@ int run(const void* A, int64_t lda, int fmt_a, const void* B, int64_t ldb, int f
   const bool any_operand = kernel == MMB200_KERNEL_AUTO && !a_hp && !shared_b &&
                            !(S > 1 && mmb::plan_has_empty_splits(mmb::make_plan(K, p.fast, S, p.scheme)));
   const bool staged_ok = (any_operand ? mmb::staged_supports(p, nfma) : mmb::staged_vector_supports(p, nfma)) && workspace &&
-                         workspace_bytes >= mmb::staged_workspace_bytes(M, N, K, S, false, shared_b != nullptr) &&
+                         workspace_bytes >= mmb::staged_workspace_bytes(M, N, K, S, false, shared_b != nullptr, alu) &&
                          !(reinterpret_cast<uintptr_t>(workspace) & 127);
   if (shared_b && !staged_ok) return MMB200_ERR_UNSUPPORTED;      // only the staged kernels read a shared B area
   if (kernel == MMB200_KERNEL_FAST && !direct_ok && !staged_ok) return MMB200_ERR_UNSUPPORTED;
@@ -291,7 +292,9 @@ int mmb200_scaled_mm(const void* A, int64_t lda, int fmt_a, const void* B, int64
              scale_result, 1, 1, kernel, stream);
 }
 
-size_t mmb200_workspace_status_offset(int M, int N, int K, int S) { return mmb::staged_status_offset(M, N, K, S); }
+size_t mmb200_workspace_status_offset(int M, int N, int K, int S) {
+  return K > 0 && S >= 1 ? mmb::staged_status_offset(M, N) : 0;
+}
 
 int mmb200_workspace_status(const void* workspace, int M, int N, int K, int S, void* stream) {
   if (M < 0 || N < 0 || K < 0 || S < 1) return MMB200_ERR_BAD_ARG;
@@ -311,8 +314,12 @@ int mmb200_probe_issue_rate(int kind, int ctas, int iters, float* sink, void* st
 
 void mmb200_test_hooks(int wait_polls, int announce_extra_bytes) { mmb::staged_test_hooks(wait_polls, announce_extra_bytes); }
 
-size_t mmb200_workspace_bytes(int M, int N, int K) { return mmb::staged_workspace_bytes(M, N, K, 1, false); }
-size_t mmb200_workspace_bytes_split(int M, int N, int K, int S) { return mmb::staged_workspace_bytes(M, N, K, S, true); }
+size_t mmb200_workspace_bytes(int M, int N, int K) {
+  return mmb::staged_workspace_bytes(M, N, K, 1, false, false, mmb::tensor_cores_off());
+}
+size_t mmb200_workspace_bytes_split(int M, int N, int K, int S) {
+  return mmb::staged_workspace_bytes(M, N, K, S, true, false, mmb::tensor_cores_off());
+}
 
 int mmb200_scaled_mm_ws(const void* A, int64_t lda, int fmt_a, const void* B, int64_t ldb, int fmt_b, void* D,
                         int64_t ldd, int out_dtype, int M, int N, int K, int nfma, int fast, int S, int scheme,
@@ -374,6 +381,7 @@ int mmb200_scaled_mm_host(const void* A, int64_t lda, int fmt_a, const void* B, 
   // GPU always has a slab whose rows have arrived (rows are independent of one another; B is copied and decoded once,
   // into a shared area). A slab on a stream of its own never waits behind another slab: with fewer streams than slabs
   // the slab queued behind the one the GPU happened to run last ran alone at the end.
+  const bool alu = mmb::tensor_cores_off();             // one answer for the sizes, the decoded B and every slab
   HostPipeline* pipe = nullptr;
   int slab_rows = M, n_slabs = 1;
   const int setting = host_pipeline_setting();
@@ -386,7 +394,7 @@ int mmb200_scaled_mm_host(const void* A, int64_t lda, int fmt_a, const void* B, 
       tile_rows = ((M + 127) / 128 + PIPELINE_MAX_SLABS - 1) / PIPELINE_MAX_SLABS;
       slabs = ((M + 127) / 128 + tile_rows - 1) / tile_rows;
     }
-    if (slabs >= 2 && mmb::staged_workspace_bytes(tile_rows * 128, N, K, S, true, true)) {
+    if (slabs >= 2 && mmb::staged_workspace_bytes(tile_rows * 128, N, K, S, true, true, alu)) {
       cudaError_t perr = host_pipeline(&pipe);
       if (perr != cudaSuccess) return cuda_fail(perr);
       slab_rows = tile_rows * 128;
@@ -396,9 +404,9 @@ int mmb200_scaled_mm_host(const void* A, int64_t lda, int fmt_a, const void* B, 
   // device staging: A, B, D, the three scales, then scratch memory of the staged kernels (one per slab, B shared)
   const size_t a_off = 0, b_off = up(a_bytes), d_off = b_off + up(b_bytes), s_off = d_off + up(d_bytes);
   const size_t sb_off = s_off + 256;
-  const size_t sb_bytes = pipe ? up(mmb::staged_shared_b_bytes(N, K)) : 0;
+  const size_t sb_bytes = pipe ? up(mmb::staged_shared_b_bytes(N, K, alu)) : 0;
   const size_t w_off = sb_off + sb_bytes;
-  const size_t w_each = staged ? up(mmb::staged_workspace_bytes(slab_rows, N, K, S, true, pipe != nullptr)) : 0;
+  const size_t w_each = staged ? up(mmb::staged_workspace_bytes(slab_rows, N, K, S, true, pipe != nullptr, alu)) : 0;
   const size_t total = w_off + w_each * (size_t)n_slabs;
   uint8_t* buf = nullptr;
   cudaMemPool_t pool = nullptr;
@@ -426,9 +434,9 @@ int mmb200_scaled_mm_host(const void* A, int64_t lda, int fmt_a, const void* B, 
       }
       err = cudaMemcpyAsync(buf + s_off, scales, sizeof(scales), cudaMemcpyHostToDevice, st);
       if (err != cudaSuccess) break;
-      rc = mmb200_scaled_mm_ws(buf + a_off, (int64_t)kpad, fmt_a, buf + b_off, (int64_t)kpad, fmt_b, buf + d_off, N,
-                               out_dtype, M, N, K, nfma, fast, S, scheme, sdev, sdev + 1,
-                               scale_result ? sdev + 2 : nullptr, kernel, w_each ? buf + w_off : nullptr, w_each, stream);
+      rc = run(buf + a_off, (int64_t)kpad, fmt_a, buf + b_off, (int64_t)kpad, fmt_b, buf + d_off, N, out_dtype, M, N, K,
+               nfma, fast, S, scheme, sdev, sdev + 1, scale_result ? sdev + 2 : nullptr, 1, 1, kernel, stream,
+               w_each ? buf + w_off : nullptr, w_each, nullptr, 0, 0, nullptr, nullptr, 0, nullptr, alu);
       if (rc != MMB200_OK) break;
       if (w_each) {                       // the staged kernels report a wait that ran out; D is then not copied back
         rc = read_status(buf + w_off, M, N, K, S, st);
@@ -452,6 +460,7 @@ int mmb200_scaled_mm_host(const void* A, int64_t lda, int fmt_a, const void* B, 
       mmb::Params pb;
       std::memset(&pb, 0, sizeof(pb));
       pb.B = buf + b_off; pb.ldb = (long long)kpad; pb.N = N; pb.K = K; pb.fmt_a = fmt_a; pb.fmt_b = fmt_b; pb.S = S;
+      pb.no_tensor_epass = alu ? 1 : 0;
       pb.shared_b = buf + sb_off;
       int launches = 0;
       err = mmb::launch_predecode_b(pb, nfma, s0, &launches);
@@ -473,7 +482,7 @@ int mmb200_scaled_mm_host(const void* A, int64_t lda, int fmt_a, const void* B, 
       if (err != cudaSuccess) break;
       rc = run(a_dev, (int64_t)kpad, fmt_a, buf + b_off, (int64_t)kpad, fmt_b, d_dev, N, out_dtype, rows, N, K, nfma,
                fast, S, scheme, sdev, sdev + 1, scale_result ? sdev + 2 : nullptr, 1, 1, kernel, sq, ws, w_each, nullptr,
-               0, 0, nullptr, nullptr, 0, buf + sb_off);
+               0, 0, nullptr, nullptr, 0, buf + sb_off, alu);
       if (rc != MMB200_OK) break;
       err = cudaMemcpy2DAsync(static_cast<uint8_t*>(D) + (size_t)m0 * (size_t)ldd * es, (size_t)ldd * es, d_dev,
                               (size_t)N * es, (size_t)N * es, (size_t)rows, cudaMemcpyDeviceToHost, sq);
@@ -490,7 +499,7 @@ int mmb200_scaled_mm_host(const void* A, int64_t lda, int fmt_a, const void* B, 
     }
     for (int i = 0; i < n_slabs && err == cudaSuccess && rc == MMB200_OK; ++i) {   // status words of the slabs' bounded waits
       const int m0 = i * slab_rows, rows = (M - m0 < slab_rows) ? M - m0 : slab_rows;
-      err = cudaMemcpyAsync(&words[i], buf + w_off + (size_t)i * w_each + mmb::staged_status_offset(rows, N, K, S, true),
+      err = cudaMemcpyAsync(&words[i], buf + w_off + (size_t)i * w_each + mmb::staged_status_offset(rows, N),
                             sizeof(int), cudaMemcpyDeviceToHost, st);
     }
   }

@@ -51,7 +51,7 @@ struct Params {
                          // themselves (set by the launcher: calls with at most 16 rows, and calls whose 128 x 128 output
                          // tiles and chains would leave most SMs idle)
   int row_groups;        // 16-row groups per 128-row tile in that case (grid z): 1 or 8
-  int no_tensor_epass;   // 1: the staged kernels keep the exponent pass on the CUDA cores (packed integers) for every pair
+  int no_tensor_epass;   // 1: the staged kernels are those of the CUDA cores, for every pair (tensor_cores_off)
   // multi-GPU assembly: the same output element is also stored at the same index of every peer_D[i] (device pointers
   // into other GPUs' memory, mapped into this process), so that every GPU ends up with the whole result
   void* peer_D[MMB200_MAX_PEERS];
@@ -314,16 +314,19 @@ bool fast_supports(const Params& p, int nfma);
 // `launches` is increased by the number of kernels launched.
 bool staged_supports(const Params& p, int nfma);            // any plan, any operands (with scratch memory), up to 65,535 tiles
 bool staged_vector_supports(const Params& p, int nfma);     // any plan, operands that 16-byte loads can read
-size_t staged_workspace_bytes(int M, int N, int K, int S, bool with_slices, bool shared_b = false);
+// `alu`: for the CUDA-core kernels, whose tiles are larger; callers ask tensor_cores_off() once and size, fill and launch by
+// that one answer.
+bool tensor_cores_off();      // $MMAEMU_B200_TC_EPASS is "0"
+size_t staged_workspace_bytes(int M, int N, int K, int S, bool with_slices, bool shared_b, bool alu);
 // Bytes of a shared B area (tile images of every 128-column group, then one int per column), and the launch that fills
-// it (p.B, p.ldb, p.N, p.K, the formats; p.shared_b = the area, 128-byte aligned).
-size_t staged_shared_b_bytes(int N, int K);
+// it (p.B, p.ldb, p.N, p.K, the formats, p.no_tensor_epass; p.shared_b = the area, 128-byte aligned).
+size_t staged_shared_b_bytes(int N, int K, bool alu);
 cudaError_t launch_predecode_b(const Params& p, int nfma, cudaStream_t stream, int* launches);
 cudaError_t launch_staged(const Params& p, int nfma, void* workspace, size_t workspace_bytes, cudaStream_t stream,
                           int* launches);
 // Byte offset, inside the scratch memory of a staged launch, of the int32 status word (0, or 1 when a bounded wait ran
-// out and the output was not written); the same with and without K slices.
-size_t staged_status_offset(int M, int N, int K, int S, bool shared_b = false);
+// out and the output was not written); the same for every plan and kind of kernel.
+size_t staged_status_offset(int M, int N);
 // Test hooks of the bounded waits (process-wide; wait_polls <= 0 and announce_extra <= 0 restore the defaults).
 void staged_test_hooks(int wait_polls, int announce_extra);
 // Text of the last CUDA runtime error seen by this thread inside the library; returns MMB200_ERR_LAUNCH.

@@ -1218,27 +1218,32 @@ cudaError_t dispatch_formats(const Params& p, int nfma, cudaStream_t stream, boo
 constexpr int SLICE_TILE_LIMIT = 74, SLICE_CTA_TARGET = 296;
 constexpr size_t SLICE_SCRATCH_LIMIT = (size_t)4 << 30;
 
+// Bytes of a decoded tile: the images of both kinds of tensor-core kernels (TileTC here, UmmaTile in kernel_umma.cu) have one
+// size.
+constexpr size_t TC_TILE = sizeof(TileTC);
+static_assert(TC_TILE == UMMA_TILE_BYTES, "one size for both kinds of tile images");
+size_t b_tile_bytes(bool alu) { return alu ? sizeof(TileB) : TC_TILE; }
+
 struct WorkspaceLayout {
-  size_t a, b, flag_a, flag_b, status, seq, tot, slot, chains, chains_bytes, total;
+  size_t flag_a, flag_b, status, a, b, seq, tot, slot, chains, chains_bytes, total;
   int tiles_m, tiles_n, k_tiles;
 };
-// Offsets of the scratch memory. The layout without K slices is a prefix of the one with them.
-WorkspaceLayout workspace_layout(int M, int N, int K, int S, bool with_slices, bool shared_b = false) {
+// Offsets of the scratch memory. The layout without K slices is a prefix of the one with them; the flags and the status word
+// come first, where neither the plan nor the kind of kernel moves them. `alu`: tiles of the CUDA-core kernels (40 and 32 KB
+// per 128 rows and 32 k instead of 16).
+WorkspaceLayout workspace_layout(int M, int N, int K, int S, bool with_slices, bool shared_b, bool alu) {
   WorkspaceLayout w;
   w.tiles_m = (M + BM - 1) / BM;
   w.tiles_n = (N + BN - 1) / BN;
   w.k_tiles = (K + KT - 1) / KT;
   const size_t tiles = (size_t)w.tiles_m * w.tiles_n;
   const size_t per_tile = (size_t)TM * TN * THREADS * sizeof(float);
-  // every staged variant must fit: tiles of the CUDA-core exponent pass (TileA / TileB) or of the tensor-core one
-  constexpr size_t A_TILE = sizeof(TileA) > sizeof(TileTC) ? sizeof(TileA) : sizeof(TileTC);
-  constexpr size_t B_TILE = sizeof(TileB) > sizeof(TileTC) ? sizeof(TileB) : sizeof(TileTC);
-  w.a = 0;
-  w.b = w.a + (size_t)w.tiles_m * w.k_tiles * A_TILE;
-  w.flag_a = w.b + (shared_b ? 0 : (size_t)w.tiles_n * w.k_tiles * B_TILE);   // B's tiles live in the shared area then
+  w.flag_a = 0;
   w.flag_b = w.flag_a + (size_t)w.tiles_m * BM * sizeof(int);
   w.status = w.flag_b + (size_t)w.tiles_n * BN * sizeof(int);
-  w.seq = w.status + 256;
+  w.a = w.status + 256;
+  w.b = w.a + (size_t)w.tiles_m * w.k_tiles * (alu ? sizeof(TileA) : TC_TILE);
+  w.seq = w.b + (shared_b ? 0 : (size_t)w.tiles_n * w.k_tiles * b_tile_bytes(alu));   // B's tiles live in the shared area then
   const bool sliceable = tiles < (size_t)SLICE_TILE_LIMIT;
   // the tile sequence (at most one entry per k-tile plus one per empty split): split plans and K slices
   w.tot = w.seq;
@@ -1291,41 +1296,40 @@ cudaError_t launch_fast(const Params& p_in, int nfma, cudaStream_t stream) {
   return dispatch_formats(p, nfma, stream, false, &launches);
 }
 
-size_t staged_workspace_bytes(int M, int N, int K, int S, bool with_slices, bool shared_b) {
-  if (M <= 0 || N <= 0 || K <= 0 || !staged_grid_ok(M, N)) return 0;
-  return workspace_layout(M, N, K, S < 1 ? 1 : S, with_slices, shared_b).total;
+bool tensor_cores_off() {
+  const char* env = std::getenv("MMAEMU_B200_TC_EPASS");
+  return env && env[0] == '0' && env[1] == 0;
 }
 
-size_t staged_status_offset(int M, int N, int K, int S, bool shared_b) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  return workspace_layout(M, N, K, S < 1 ? 1 : S, false, shared_b).status;
+size_t staged_workspace_bytes(int M, int N, int K, int S, bool with_slices, bool shared_b, bool alu) {
+  if (M <= 0 || N <= 0 || K <= 0 || !staged_grid_ok(M, N)) return 0;
+  return workspace_layout(M, N, K, S < 1 ? 1 : S, with_slices, shared_b, alu).total;
+}
+
+size_t staged_status_offset(int M, int N) {
+  if (M <= 0 || N <= 0) return 0;
+  return workspace_layout(M, N, 1, 1, false, false, false).status;
 }
 
 namespace {
 // Shared B area: tile images, then the column flags.
-size_t shared_b_flags_offset(int N, int K) {
-  const WorkspaceLayout w = workspace_layout(1, N, K, 1, false);
-  return (w.flag_a - w.b + 255) / 256 * 256;
+size_t shared_b_flags_offset(int N, int K, bool alu) {
+  return (size_t)((N + BN - 1) / BN) * ((K + KT - 1) / KT) * b_tile_bytes(alu);
 }
 }  // namespace
-size_t staged_shared_b_bytes(int N, int K) {
+size_t staged_shared_b_bytes(int N, int K, bool alu) {
   if (N <= 0 || K <= 0) return 0;
-  return shared_b_flags_offset(N, K) + ((size_t)((N + BN - 1) / BN) * BN * sizeof(int) + 255) / 256 * 256;
+  return shared_b_flags_offset(N, K, alu) + (size_t)((N + BN - 1) / BN) * BN * sizeof(int);
 }
 
 cudaError_t launch_predecode_b(const Params& p_in, int nfma, cudaStream_t stream, int* launches) {
   Params p = p_in;
   if (!p.shared_b || (reinterpret_cast<uintptr_t>(p.shared_b) & 127)) return cudaErrorInvalidValue;
-  const WorkspaceLayout w = workspace_layout(1, p.N, p.K, 1, false);
-  p.tiles_m = 0; p.tiles_n = w.tiles_n; p.k_tiles = w.k_tiles;
+  p.tiles_m = 0; p.tiles_n = (p.N + BN - 1) / BN; p.k_tiles = (p.K + KT - 1) / KT;
   p.ws_b = p.shared_b;
-  p.ws_flag_b = reinterpret_cast<int*>(p.shared_b + shared_b_flags_offset(p.N, p.K));
+  p.ws_flag_b = reinterpret_cast<int*>(p.shared_b + shared_b_flags_offset(p.N, p.K, p.no_tensor_epass != 0));
   p.only_b = 1;
-  {
-    const char* env = std::getenv("MMAEMU_B200_TC_EPASS");
-    if (env && env[0] == '0' && env[1] == 0) p.no_tensor_epass = 1;
-  }
-  cudaError_t err = cudaMemsetAsync(p.ws_flag_b, 0, (size_t)w.tiles_n * BN * sizeof(int), stream);
+  cudaError_t err = cudaMemsetAsync(p.ws_flag_b, 0, (size_t)p.tiles_n * BN * sizeof(int), stream);
   if (err != cudaSuccess) return err;
   if (p.S <= 1 && umma_supports(p)) return launch_umma(p, nfma, stream, launches);   // as launch_staged decides for a shared B area
   return dispatch_formats(p, nfma, stream, true, launches);
@@ -1342,15 +1346,11 @@ void staged_test_hooks(int wait_polls, int announce_extra) {
 cudaError_t launch_staged(const Params& p_in, int nfma, void* workspace, size_t workspace_bytes, cudaStream_t stream,
                           int* launches) {
   Params p = p_in;
-  const bool shared_b = p.shared_b != nullptr;
+  const bool shared_b = p.shared_b != nullptr, alu = p.no_tensor_epass != 0;
   if (shared_b && (reinterpret_cast<uintptr_t>(p.shared_b) & 127)) return cudaErrorInvalidValue;
-  WorkspaceLayout w = workspace_layout(p.M, p.N, p.K, p.S, false, shared_b);
+  WorkspaceLayout w = workspace_layout(p.M, p.N, p.K, p.S, false, shared_b, alu);
   if (!workspace || workspace_bytes < w.total || (reinterpret_cast<uintptr_t>(workspace) & 127)) return cudaErrorInvalidValue;
   if (!staged_grid_ok(p.M, p.N)) return cudaErrorInvalidValue;
-  {
-    const char* env = std::getenv("MMAEMU_B200_TC_EPASS");         // "0": the packed-integer exponent pass for every pair
-    if (env && env[0] == '0' && env[1] == 0) p.no_tensor_epass = 1;
-  }
   const Plan plan = make_plan(p.K, p.fast, p.S, p.scheme);
   // K slices: few output tiles, a plan with more than one chain, and scratch memory for the chain results
   p.slices = 1;
@@ -1358,7 +1358,7 @@ cudaError_t launch_staged(const Params& p_in, int nfma, void* workspace, size_t 
   p.row_groups = 1;
   std::vector<uint32_t> seq;
   {
-    const WorkspaceLayout wx = workspace_layout(p.M, p.N, p.K, p.S, true, shared_b);
+    const WorkspaceLayout wx = workspace_layout(p.M, p.N, p.K, p.S, true, shared_b, alu);
     const long long tiles = (long long)w.tiles_m * w.tiles_n;
     // the 16-row kernels decode A themselves, so the quantise prologue (part of the pre-decode pass) excludes them
     const long long tiles16 = (long long)w.tiles_n * ((p.M + 15) / 16);
@@ -1393,7 +1393,6 @@ cudaError_t launch_staged(const Params& p_in, int nfma, void* workspace, size_t 
     // fast, 16 products: 298 us on 16-row CTAs, 392 on tiles).
     const long long sms = sm_count();
     const bool umma_any = umma_supports(p) && !(shared_b && p.S > 1), umma_whole = umma_any && p.S == 1;
-    const bool alu = p.no_tensor_epass != 0;
     const bool one_sum = nfma == 16 || (p.fmt_a == MMB200_FMT_E4M3 && p.fmt_b == MMB200_FMT_E4M3);
     const double UMMA = nfma == 16 ? 2.2 : (one_sum ? 1.3 : 1.65), MMA = alu ? 8.0 : (nfma == 16 ? 3.3 : 3.0);
     const double ROWS16 = alu ? 0.26 * MMA : (nfma == 32 ? 0.95 : 1.25);
@@ -1451,7 +1450,7 @@ cudaError_t launch_staged(const Params& p_in, int nfma, void* workspace, size_t 
   p.ws_flag_b = reinterpret_cast<int*>(base + w.flag_b);
   if (shared_b) {                                                // decoded by launch_predecode_b
     p.ws_b = p.shared_b;
-    p.ws_flag_b = reinterpret_cast<int*>(p.shared_b + shared_b_flags_offset(p.N, p.K));
+    p.ws_flag_b = reinterpret_cast<int*>(p.shared_b + shared_b_flags_offset(p.N, p.K, alu));
   }
   p.only_b = 0;
   p.byte_loads = vector_loads(p) ? 0 : 1;
@@ -1459,7 +1458,7 @@ cudaError_t launch_staged(const Params& p_in, int nfma, void* workspace, size_t 
   p.plan_group = plan.group;
   p.wait_polls = g_wait_polls.load();
   p.test_announce_extra = g_announce_extra.load();
-  cudaError_t err = cudaMemsetAsync(base + w.flag_a, 0, w.seq - w.flag_a, stream);   // row flags and status word
+  cudaError_t err = cudaMemsetAsync(base + w.flag_a, 0, w.a - w.flag_a, stream);     // row flags and status word
   if (err != cudaSuccess) return err;
   if (p.S > 1 || p.slices > 1) {
     p.seq_len = plan_sequence(plan, p.K, nullptr);

@@ -40,7 +40,7 @@ constexpr uint32_t R_ZERO = 0x3FC00000u;       // 1.5: an offset accumulator tha
 struct UmmaTile {
   uint4 c[8][128];
 };
-static_assert(sizeof(UmmaTile) == 16384, "tile layout");
+static_assert(sizeof(UmmaTile) == UMMA_TILE_BYTES, "tile layout");
 template <int NW>
 struct UmmaStage { UmmaTile a, b[NW / 64]; };
 template <int NW, bool PARTS>

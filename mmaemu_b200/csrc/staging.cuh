@@ -10,6 +10,7 @@ namespace mmb {
 namespace {
 
 constexpr int BM = 128, BN = 128, KT = 32, THREADS = 256;
+constexpr size_t UMMA_TILE_BYTES = 16384;      // operand image of 128 rows and 32 k for the tcgen05 kernels
 
 // The power base of a format pair's tensor-core exponent pass (2^8, 2^5 or 2^4 per unit of exponent): see
 // block_strip_mma and fast_math.cuh.

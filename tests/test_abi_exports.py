@@ -65,6 +65,21 @@ def test_status_codes_and_argument_checks_without_a_device(lib):
     assert lib.mmb200_launch_count() == 0
 
 
+def test_scratch_memory_is_what_the_kernels_use(lib, monkeypatch):
+    """A tile image takes 16 KB per 128 rows and 32 k; the CUDA-core kernels' tiles 40 KB of A and 32 KB of B. The status word's
+    place depends on neither."""
+    M, N, K = 1000, 300, 100                              # 8 x 3 tiles, 4 k-tiles
+    rest = 4 * 128 * (8 + 3) + 256
+    monkeypatch.delenv("MMAEMU_B200_TC_EPASS", raising=False)
+    off = lib.mmb200_workspace_status_offset(M, N, K, 1)
+    tiles = lib.mmb200_workspace_bytes(M, N, K) - rest
+    assert (8 + 3) * 4 * 16384 <= tiles < (8 + 3) * 4 * 16384 + 1024
+    monkeypatch.setenv("MMAEMU_B200_TC_EPASS", "0")
+    tiles = lib.mmb200_workspace_bytes(M, N, K) - rest
+    assert 4 * (8 * 40960 + 3 * 32768) <= tiles < 4 * (8 * 40960 + 3 * 32768) + 1024
+    assert lib.mmb200_workspace_status_offset(M, N, K, 1) == off
+
+
 def test_shapes_beyond_the_grid_of_the_scratch_memory_kernels_ask_for_no_scratch(lib):
     """65,535 tiles of 128 rows or columns are the most that one launch takes; the integer kernel serves larger shapes."""
     most = 65535 * 128
