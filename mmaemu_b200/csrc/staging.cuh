@@ -120,7 +120,8 @@ __device__ __forceinline__ void decode4(uint32_t& w, uint32_t& h01, uint32_t& h2
     const uint32_t nonzero = __hne2_mask(v, __float2half2_rn(0.0f));
     const uint32_t x = *reinterpret_cast<const uint32_t*>(&m) & 0x7C007C00u;
     uint32_t lane;                                                         // field << 7 in both halves
-    if (MUL == 8) lane = x;                                                // bias 72 = 8 * OFF
+    static_assert(MUL != 8 || (int)fm::POW8_BIAS == 8 * OFF, "E4M3: 8 times the fp16 field is the power's field");
+    if (MUL == 8) lane = x;                                                // OFF and the bias cancel
     else if (MUL == 5) lane = (x >> 3) * 5u + (uint32_t)((int)fm::POW5_BIAS - 5 * OFF) * 0x00800080u;
     else lane = (x >> 1) + (uint32_t)((int)(IS_A ? fm::POW4_BIAS_A : fm::POW4_BIAS_B) - 4 * OFF) * 0x00800080u;
     return lane & nonzero;
