@@ -70,3 +70,17 @@ def test_operands_without_16_byte_loads(M, N, K, fmts, fast):
     for preset in (16, 32):
         same("accumulate", codes(rng, M, K, fmts[0]), codes(rng, N, K, fmts[1]), fmt_a=fmts[0], fmt_b=fmts[1], preset=preset,
              fast=fast)
+
+
+@pytest.mark.parametrize("kernel", ("staged", "staged-rows"))
+@pytest.mark.parametrize("ld_pad", (1, 8, 16))
+@pytest.mark.parametrize("M,N,K", ((16, 130, 48), (150, 129, 416)))
+def test_odd_leading_dimensions(M, N, K, ld_pad, kernel):
+    """K a multiple of 16 but rows that start anywhere (ld_pad 16: the 16-byte loads of the same call)."""
+    import gpu_runner
+    rng = np.random.default_rng(K + ld_pad)
+    a, b = codes(rng, M, K, "e5m2"), codes(rng, N, K, "e4m3")
+    for fast in (True, False):
+        got, want = (gpu_runner.scaled_mm(a, b, 0.37, 2.5, fmt_a="e5m2", out="float32", preset=32, fast=fast, kernel=k, ld_pad=ld_pad)
+                     for k in (kernel, "integer"))
+        assert np.array_equal(got, want)
