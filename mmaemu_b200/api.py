@@ -326,6 +326,8 @@ def _workspace(L, kernel: str, a_ptr, lda, b_ptr, ldb, M, N, K, nfma, S, scheme,
     try:
         ws = torch.empty(n, dtype=torch.uint8, device=device)
     except torch.OutOfMemoryError:
+        if kernel != "auto":
+            raise                            # a request for the fast kernels by name
         return None, None, 0                 # the kernels that need no scratch memory serve every call, more slowly
     return ws, ws.data_ptr(), n
 

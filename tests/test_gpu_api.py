@@ -226,6 +226,9 @@ def test_a_call_without_memory_left_for_scratch_is_served(K, monkeypatch):
         S, scheme = (1, "none") if splitk == 1 else splitk
         assert np.array_equal(bits(acc), oracle.accumulate(a, b, preset="hopper", fast=fast, S=S, scheme=scheme))
     assert refused
+    if K % 16 == 0:                                       # a request for the fast kernels by name says what is missing
+        with pytest.raises(torch.OutOfMemoryError):
+            mm.accumulate(ta, tb, use_fast_accum=True, profile="hopper", splitk=(2, "contiguous"), backend="cuda:b200-fast")
 
 
 def test_backend_object_chain_fn():
