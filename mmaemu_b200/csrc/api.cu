@@ -107,8 +107,8 @@ int run(const void* A, int64_t lda, int fmt_a, const void* B, int64_t ldb, int f
   // fast kernels: every plan with enough scratch memory (staged), unsplit plans without; else the integer kernel
   const bool direct_ok = mmb::fast_supports(p, nfma);
   // A request for the fast kernels by name, the quantise prologue and a shared B area keep to operands that 16-byte loads
-  // can read; the automatic choice takes any operand to the staged kernels (517 x 1003 x 2001: 75 us of kernels, 592 us on the
-  // integer kernel) -- but not plans with empty splits, which their walker visits one by one at several us each (300 x 300 x 33
+  // can read; the automatic choice takes any operand to the staged kernels (517 x 1003 x 2001: 75 us on them, 592 us on the
+  // integer kernel), but not plans with empty splits, which their walker visits one by one at several us each (300 x 300 x 33
   // split in five: 84 us, 45 us on the integer kernel).
   const bool any_operand = kernel == MMB200_KERNEL_AUTO && !a_hp && !shared_b &&
                            !(S > 1 && mmb::plan_has_empty_splits(mmb::make_plan(K, p.fast, S, p.scheme)));
@@ -374,6 +374,7 @@ int mmb200_scaled_mm_host(const void* A, int64_t lda, int fmt_a, const void* B, 
   const size_t kpad = ((size_t)K + 15) / 16 * 16;       // dense device copies with a 16-byte aligned row stride
   const size_t a_bytes = (size_t)M * kpad, b_bytes = (size_t)N * kpad, d_bytes = (size_t)M * N * es;
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+  // (a K that is no multiple of 16 stays on the integer kernel here)
   const bool staged = K > 0 && K % 16 == 0 && S >= 1 && S <= MMB200_MAX_SPLITS && kernel != MMB200_KERNEL_INTEGER &&
                       (nfma == MMB200_PRESET_ADA || nfma == MMB200_PRESET_HOPPER);
   // Row slabs: with enough work the rows of A are cut into slabs, each on an internal stream of its own (copy of its

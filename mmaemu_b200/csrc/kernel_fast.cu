@@ -812,7 +812,7 @@ __global__ void __launch_bounds__(THREADS) predecode_tc_kernel(const __grid_cons
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// The staged kernels: decoded tiles arrive by bulk asynchronous copies into a two-stage ring.
+// The staged kernels: decoded tiles arrive by bulk asynchronous copies into a ring of stages.
 template <bool TC> struct StageOf { TileA a; TileB b; };
 template <> struct StageOf<true> { TileTC a, b; };
 template <bool TC> constexpr int STAGES = TC ? 4 : 2;   // 32 KB per stage with the tensor-core tiles, 72 KB otherwise

@@ -13,16 +13,22 @@
 //
 // Tiles: 128 rows, two halves of NW columns each, so that the tensor cores run one half's products while the warps of the
 // other half compute. An MMA of 64 columns takes as long as one of 128 (95 and 97 cycles; 161 with 256), so NW = 128 is
-// the better shape where the output has enough 256-column tiles and TMEM holds them: fast accumulation, one exponent sum
-// per block. NW = 64 otherwise, and for K slices.
+// the better shape where the output has enough 256-column tiles and TMEM holds R and the exponent sums: one sum per block.
+// NW = 64 otherwise, and for K slices.
 //
 // TMEM (512 columns x 128 lanes of 32 bits): offset accumulators R in columns 0 .. 2 NW - 1, exponent sums behind them (two
-// sets with NW = 64), the running sums of slow accumulation in the last 128. Nothing is kept in registers between blocks.
+// sets with NW = 64). The running sums of slow accumulation take the last 128 columns with NW = 64; with NW = 128 TMEM is full
+// and they live in shared memory (128 KB), which leaves two stages of operand images instead of four. Nothing is kept in
+// registers between blocks.
 //
 // Roles: 16 warps run the scalar steps (warp w: lanes 32 (w % 4) .., a quarter w / 4 of the columns); one thread issues the
-// MMAs, one thread the bulk copies of the operand images. Every wait is bounded. Per output and block the warps issue 4
-// instructions for the half-rate INT pipe and 2 FMAs beside TMEM loads and stores (one column per cycle each): about 8 cycles
-// per scheduler and 32 outputs, which bounds the kernel.
+// MMAs, one thread the bulk copies of the operand images. Every wait is bounded.
+//
+// What bounds it. Per output and block the warps issue 4 instructions for the half-rate INT pipe and 2 FMAs beside TMEM loads
+// and stores (one column per cycle each): 8 cycles per scheduler and 32 outputs at best. Measured: 13 with fast accumulation
+// (8192 x 24576 x 8192, 18.1 ms), 18 with slow (4096-cube, 1.21 ms; INT pipe 61 % busy). The rest is the latency from a half's
+// stores of R over its MMAs to its next loads, which the other half covers only in part, and with slow accumulation the chain
+// end, a pass over TMEM of its own every 128 k (0.92 ms without it on the same tiles).
 #include <atomic>
 
 #include "staging.cuh"
