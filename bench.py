@@ -51,11 +51,13 @@ STRONG = dict(name="cfg5_recipe_16384x16384x8192", profile="hopper", M=16384, N=
 # (smsp__inst_executed.sum * 32 / (M*N*K), profiles/): keyed by (kernel, products per block, accumulation). A workload
 # whose kernel has no capture gets no issue-slot roofline (null), never another kernel's constant.
 INST_PER_MAC = {("umma_kernel", 32, "slow"): 0.345,             # 2048 cube, profiles/umma_kernel_hopper_e4m3_2048cube.md
+                ("umma_kernel, K slices", 32, "slow"): 0.470,   # e5m2 x e4m3, profiles/sliced_kernels_hopper_e5m2xe4m3_128x4096x16384.md
+                ("staged_tc_kernel, 16 rows per CTA", 32, "slow"): 1.648,   # e5m2 x e4m3, profiles/few_rows_kernel_hopper_e5m2xe4m3_16x4096x8192.md
                 ("staged_kernel", 32, "slow"): 3.16,           # 2048 cube e5m2 x e4m3 with MMAEMU_B200_TC_EPASS=0, profiles/staged_kernel_hopper_e5m2xe4m3_2048cube.md
                 ("fast_kernel", 32, "slow"): 3.37,             # 2048 cube, profiles/fast_kernel_hopper_e4m3_2048cube.md
                 ("integer_kernel", 32, "slow"): 8.56}           # 2048 cube, profiles/integer_kernel_hopper_e4m3_2048cube.md
-# DRAM bytes per launch of the main kernel by workload, from one-pass ncu captures at full size: none of the present kernels.
-DRAM_TRAFFIC = {}
+# DRAM bytes per launch of the main kernel by workload, from one-pass ncu captures at full size.
+DRAM_TRAFFIC = {("umma_kernel", 32, "slow", 4096, 4096, 4096): 275076096 + 24301056}
 
 
 # ---------------------------------------------------------------------------------------------------------------
@@ -314,6 +316,9 @@ def kernel_of(cfg, S=1) -> str:
     """Name of the main kernel the automatic choice runs for a configuration (with scratch memory)."""
     if cfg["M"] <= 16:
         return "staged_tc_kernel, 16 rows per CTA"
+    tiles = -(-cfg["M"] // 128) * -(-cfg["N"] // 128)
+    if tiles < 74 and (S > 1 or not cfg["fast"]) and (cfg["fa"], cfg["fb"]) != ("e5m2", "e5m2"):
+        return "umma_kernel, K slices"
     return "staged_tc_kernel" if (cfg["fa"], cfg["fb"]) == ("e5m2", "e5m2") else "umma_kernel"
 
 
@@ -459,7 +464,8 @@ def other_configs(mm, oracle, timer, dev, issue_peak_t):
     finally:
         os.environ.pop("MMAEMU_B200_ROW_GROUPS", None)
     out[c["name"]]["ms_without_row_groups"] = off["ms"]
-    out[c["name"]]["kernel"] = "staged_tc_kernel, 16 rows per CTA (row groups)"
+    for name in (c["name"], "cfg1_ada_256cube", "cfg3_hopper_128x128x16384"):
+        out[name]["kernel"] = "staged_tc_kernel, 16 rows per CTA (row groups)"
     # 4: FP8 projection stack, hopper-te, amax-derived scales
     for i, (N, K) in enumerate([(5760, 1920), (1920, 1920), (24576, 8192)]):
         M = 8192

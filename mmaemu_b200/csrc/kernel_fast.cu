@@ -354,7 +354,7 @@ __device__ __forceinline__ uint32_t word_of(const uint4& w, int q) { return q ==
 //
 // Per 16 x 8 outputs and 32 k: 8 + 2 mma.sync (918 multiply-adds per clock and SM measured, nominally 1,024), the operand
 // moves that put each word into both k positions, and six CUDA-core instructions per output. Measured on the 16-row kernel
-// (16 x 4096 x 8192, 58 us): issue slots 53 % used, tensor pipe 17 %, so issue and the latency of the chain of dependent
+// (16 x 4096 x 8192, 57 us): issue slots 53 % used, tensor pipe 20 %, so issue and the latency of the chain of dependent
 // instructions bound it, not the tensor pipe. A block of scalar fma.rz plus the floor -> truncation fix took 81 instructions
 // per output: 4096-cube 7.2 -> 2.8 ms with this step on 128-row tiles.
 template <int NFMA, int FA, int FB, int I0, int MI, int J0, int NI, class TA_>
